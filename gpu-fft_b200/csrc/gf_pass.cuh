@@ -451,7 +451,7 @@ inline const char* kind_name(int fwd) { return fwd ? "fwd" : "inv"; }
 // more threads are in flight than with 4096-element tiles. Load and store
 // variants are compile-time, so their selection costs nothing per element.
 // ---------------------------------------------------------------------------
-constexpr int COL_MAX_L = 4;
+constexpr int COL_MAX_L = 5;
 constexpr int COL_THREADS = 128;
 
 // Column `idx` (over all batch entries) of the pass; no shared memory, no
@@ -536,43 +536,142 @@ __device__ __forceinline__ void col_pass_body(const PassArgs<T>& a, long long id
     }
 }
 
+// Two lanes per column (l and l ^ 16 of a warp, half hb = bit 4 of the lane):
+// lane half hb holds the rows i = 2q + hb. Every stage with span >= 2 pairs rows
+// of one parity in the lane; the span-1 stage exchanges through
+// __shfl_xor_sync. Half the registers per thread of a column on one lane: 32-point
+// FP64 columns would need 128 for their data alone.
+template <typename T> __device__ __forceinline__ cx<T> shfl_half(cx<T> v)
+{
+    return mk<T>(__shfl_xor_sync(0xffffffffu, v.x, 16), __shfl_xor_sync(0xffffffffu, v.y, 16));
+}
+template <typename T, bool FWD, int L, int IK, int OK>
+__device__ __forceinline__ void col_pair_body(const PassArgs<T>& a, long long idx)
+{
+    constexpr int H = 1 << (L - 1);
+    const int m = a.geo.m, s0 = a.geo.s0;
+    const int lc = m - s0 - L; // log2 columns per group
+    const int hb = (int)((idx >> 4) & 1);
+    const long long col = ((idx >> 5) << 4) + (idx & 15);
+    // the last warp may hold columns beyond the batch: their lanes (both halves)
+    // read row 0 and store nothing
+    const long long bq = col >> (m - L);
+    const bool ok = bq < a.batch;
+    const long long b = ok ? bq : 0;
+    const long long r = col & ((1LL << (m - L)) - 1);
+    const long long g = r >> lc;
+    const long long C = 1LL << lc;
+    const long long j0 = (g << (m - s0)) + (r & (C - 1)) + hb * C;
+    cx<T> x[H];
+#pragma unroll
+    for (int q = 0; q < H; q++) x[q] = load_elem<T>(a, IK, b, j0 + 2 * q * C);
+#pragma unroll
+    for (int k = 0; k < L; k++)
+    {
+        const int u = FWD ? k : L - 1 - k; // stage s0 + u
+        const cx<T>* tw = a.table + (a.geo.neg ? (1LL << (s0 + u)) : 0LL) + (g << u);
+        if (u == L - 1)
+        {
+#pragma unroll
+            for (int q = 0; q < H; q++)
+            {
+                const cx<T> wt = ldg<T>(tw + q);
+                if (FWD)
+                {
+                    // half 0 sends U, half 1 sends V w
+                    const cx<T> mine = hb ? cmul<T>(x[q], wt) : x[q];
+                    const cx<T> other = shfl_half<T>(mine);
+                    x[q] = hb ? csub<T>(other, mine) : cadd<T>(mine, other);
+                }
+                else
+                {
+                    const cx<T> other = shfl_half<T>(x[q]);
+                    x[q] = hb ? cmul<T>(csub<T>(other, x[q]), wt) : cadd<T>(x[q], other);
+                }
+            }
+            continue;
+        }
+        const int h = 1 << (L - 2 - u);
+#pragma unroll
+        for (int q = 0; q < H; q++)
+        {
+            if (q & h) continue;
+            const cx<T> wt = ldg<T>(tw + (q >> (L - 1 - u)));
+            if (FWD)
+                ct_bfly<T>(x[q], x[q + h], wt);
+            else
+                gs_bfly<T>(x[q], x[q + h], wt);
+        }
+    }
+    if (!ok) return;
+#pragma unroll
+    for (int q = 0; q < H; q++) store_elem<T>(a, OK, b, j0 + 2 * q * C, x[q]);
+}
+
 // The column passes wait on global loads (one column's points and twiddles
 // per thread): eight-point double columns are compiled for eight CTAs per SM
-// (64 registers) so that more loads are in flight.
-template <typename T, int L> constexpr int col_min_blocks() { return (sizeof(T) == 8 && L <= 3) ? 8 : 1; }
+// (64 registers) so that more loads are in flight; so are sixteen-point ones on
+// two lanes, and 32-point columns for four (FP64) or six.
+template <typename T, int L, bool PAIR> constexpr int col_min_blocks()
+{
+    if (PAIR) return L <= 4 ? 8 : sizeof(T) == 8 ? 4 : 6;
+    return (sizeof(T) == 8 && L <= 3) ? 8 : 1;
+}
 
-template <typename T, bool FWD, int L, int IK, int OK>
-__global__ void __launch_bounds__(COL_THREADS, col_min_blocks<T, L>()) col_pass_kernel(const PassArgs<T> a)
+template <typename T, bool FWD, int L, int IK, int OK, bool PAIR>
+__global__ void __launch_bounds__(COL_THREADS, col_min_blocks<T, L, PAIR>()) col_pass_kernel(const PassArgs<T> a)
 {
     pdl_begin(); // before any global-memory access (programmatic launch)
-    col_pass_body<T, FWD, L, IK, OK>(a, (long long)blockIdx.x * COL_THREADS + threadIdx.x);
+    const long long idx = (long long)blockIdx.x * COL_THREADS + threadIdx.x;
+    if constexpr (PAIR)
+        col_pair_body<T, FWD, L, IK, OK>(a, idx);
+    else
+        col_pass_body<T, FWD, L, IK, OK>(a, idx);
 }
 
 // Launch the column form when a kernel for (in_kind, out_kind) is compiled:
 // forward first passes (any load, complex store) and inverse last passes
 // (complex load, any store). Returns -1 when the pair has no column kernel.
+// Two lanes per column: always at 32 points; in FP64 at 16 points once that
+// fills the SMs twice (N = 2^16, batch 256, forward: 94.8 -> 87.1 us; below it one
+// lane per column leaves the next launch more room: N = 2^17, batch 9: 26.8
+// against 24.7 us for the product). The 32-point FP64 forward of complex rows stays
+// with the 4096-point tile (N = 2^17, 60 rows: 50.3 against 57.6 us).
 template <typename T, bool FWD, int L>
 static inline int launch_col_pass(const PassArgs<T>& a, cudaStream_t s)
 {
-    const long long threads = a.batch << (a.geo.m - L);
-    const unsigned blocks = (unsigned)((threads + COL_THREADS - 1) / COL_THREADS);
-    auto go = [&](auto kern) {
+    const long long cols = a.batch << (a.geo.m - L);
+    if (cols > 0x3fffffffLL * COL_THREADS) return -1;
+    auto launch = [&](auto kern, long long threads) {
+        const unsigned blocks = (unsigned)((threads + COL_THREADS - 1) / COL_THREADS);
         GF_TRACE(tr, pass_alg_bytes(a), s, "col_pass<%s,%s,L%d,in%d,out%d>", sizeof(T) == 4 ? "f32" : "f64",
                  kind_name(FWD), L, a.in_kind, a.out_kind);
         return launch_k(kern, blocks, COL_THREADS, 0, s, a);
+    };
+    auto go = [&]<int IK, int OK>() -> int {
+        if constexpr (L == 5 && FWD && sizeof(T) == 8 && (IK == IN_CPX || IK == IN_CPX2)) return -1;
+        else if constexpr (L == 5) return launch(col_pass_kernel<T, FWD, L, IK, OK, true>, 2 * cols);
+        else
+        {
+            if constexpr (L == 4 && sizeof(T) == 8)
+            {
+                if (cols >= 1024LL * sm_count()) return launch(col_pass_kernel<T, FWD, L, IK, OK, true>, 2 * cols);
+            }
+            return launch(col_pass_kernel<T, FWD, L, IK, OK, false>, cols);
+        }
     };
     if constexpr (FWD)
     {
         if (a.out_kind != OUT_CPX) return -1;
         switch (a.in_kind)
         {
-        case IN_CPX: return go(col_pass_kernel<T, true, L, IN_CPX, OUT_CPX>);
-        case IN_REAL: return go(col_pass_kernel<T, true, L, IN_REAL, OUT_CPX>);
-        case IN_FOLD: return go(col_pass_kernel<T, true, L, IN_FOLD, OUT_CPX>);
-        case IN_FOLD2: return go(col_pass_kernel<T, true, L, IN_FOLD2, OUT_CPX>);
-        case IN_LIN2: return go(col_pass_kernel<T, true, L, IN_LIN2, OUT_CPX>);
-        case IN_VJP3: return go(col_pass_kernel<T, true, L, IN_VJP3, OUT_CPX>);
-        case IN_CPX2: return go(col_pass_kernel<T, true, L, IN_CPX2, OUT_CPX>);
+        case IN_CPX: return go.template operator()<IN_CPX, OUT_CPX>();
+        case IN_REAL: return go.template operator()<IN_REAL, OUT_CPX>();
+        case IN_FOLD: return go.template operator()<IN_FOLD, OUT_CPX>();
+        case IN_FOLD2: return go.template operator()<IN_FOLD2, OUT_CPX>();
+        case IN_LIN2: return go.template operator()<IN_LIN2, OUT_CPX>();
+        case IN_VJP3: return go.template operator()<IN_VJP3, OUT_CPX>();
+        case IN_CPX2: return go.template operator()<IN_CPX2, OUT_CPX>();
         default: return -1;
         }
     }
@@ -581,10 +680,10 @@ static inline int launch_col_pass(const PassArgs<T>& a, cudaStream_t s)
         if (a.in_kind != IN_CPX) return -1;
         switch (a.out_kind)
         {
-        case OUT_CPX: return go(col_pass_kernel<T, false, L, IN_CPX, OUT_CPX>);
-        case OUT_REAL: return go(col_pass_kernel<T, false, L, IN_CPX, OUT_REAL>);
-        case OUT_UNFOLD: return go(col_pass_kernel<T, false, L, IN_CPX, OUT_UNFOLD>);
-        case OUT_RE2: return go(col_pass_kernel<T, false, L, IN_CPX, OUT_RE2>);
+        case OUT_CPX: return go.template operator()<IN_CPX, OUT_CPX>();
+        case OUT_REAL: return go.template operator()<IN_CPX, OUT_REAL>();
+        case OUT_UNFOLD: return go.template operator()<IN_CPX, OUT_UNFOLD>();
+        case OUT_RE2: return go.template operator()<IN_CPX, OUT_RE2>();
         default: return -1;
         }
     }

@@ -21,6 +21,7 @@
 // sincospi in double precision (then rounded to float for the f32 path).
 #include "gf_fused.cuh"
 #include "gf_fused_r8.cuh"
+#include "gf_tile.cuh"
 
 #include <atomic>
 
@@ -166,19 +167,56 @@ template <typename T, bool SINGLE> static int launch_fused(const FusedArgs<T>& a
     return dispatch_int<1, EBITS>(a.geo.m, [&]<int LL>() { return launch_fused_shape<T, LL, true>(a, ctas, s); });
 }
 
+// Pass plan of a wave of w products with 2^m-point transforms (m > 12): the
+// tile kernel's (m - 11 column stages, eleven on 2048-point tiles), or the
+// 4096-point middle pass. Waves of fewer than two tiles per SM leave the tile
+// kernel's CTAs too few to overlap: they take the middle pass.
+template <typename T> static Plan product_plan(int m, long long w)
+{
+    Plan p = make_plan(m);
+    if (m - tile::LT > COL_MAX_L || (w << (m - tile::LT)) < 2LL * sm_count()) return p;
+    if (sizeof(T) == 8 && !g_f64_middle_r8.load(std::memory_order_relaxed)) return p;
+    p.L[0] = m - tile::LT;
+    p.L[1] = tile::LT;
+    return p;
+}
+
+// The middle of a wave of products whose spectra are in f.ws (f.batch rows of
+// A, then of B): the product's spectra replace A's.
+template <typename T> static int launch_middle(FusedArgs<T>& f, const Plan& p, int m, cudaStream_t s)
+{
+    const long long M = 1LL << m;
+    if (p.L[1] == tile::LT)
+    {
+        TileArgs<T> a{};
+        a.park = f.ws + f.batch * M;
+        a.in[0] = f.ws;
+        a.out[0] = f.ws;
+        a.roots = f.roots;
+        a.m = m;
+        return launch_tile_product<T, TILE_MUL>(a, f.batch << (m - tile::LT), s);
+    }
+    long long ctas = 0;
+    f.geo = pass_geo(p, 1, m, 0, f.batch, &ctas);
+    return launch_fused<T, false>(f, ctas, s);
+}
+
 constexpr int NATIVE_MIN_NPOWER = 2;
 constexpr int NATIVE_MAX_NPOWER = 22; // two-pass plans: M = N/2 <= 2^21
-// Recommended wave: 80 MiB of spectra (then rounded to whole waves of the SMs).
-// Measured at N = 2^16 (1 MiB of spectra per product), batch 256: waves of
-// 37 / 74 / 256 products run 718k / 770k / 750k products/s.
+// Recommended wave, then rounded to whole waves of the SMs. Rings of the tile
+// kernel: up to 320 MiB of spectra, as every launch ends in a partial wave of CTAs
+// (N = 2^16, 1 MiB per product, batch 256, FP64: 74 / 111 / 256 products per wave
+// run 252 / 252 / 241 us). Larger rings keep 80 MiB (the 4096-point middle pass at
+// N = 2^16: 37 / 74 / 256 products ran 290 / 286 / 302 us).
 constexpr size_t WAVE_TARGET_BYTES = 80ull << 20;
+constexpr size_t WAVE_TILE_BYTES = 320ull << 20;
 
 static long long wave_products(int n_power, long long batch, size_t cx_bytes)
 {
     const int m = n_power - 1;
     if (m <= EBITS) return batch;
     const size_t per = 2 * ((size_t)1 << m) * cx_bytes;
-    long long w = (long long)(WAVE_TARGET_BYTES / per);
+    long long w = (long long)((m - tile::LT <= COL_MAX_L ? WAVE_TILE_BYTES : WAVE_TARGET_BYTES) / per);
     if (w < 1) w = 1;
     w = round_wave(w, ((long long)1 << m) / ECTA);
     return w < batch ? w : batch;
@@ -230,10 +268,10 @@ static int negacyclic_mul(const T* a, const T* b, T* c, int n_power, int batch, 
     else
         W = round_wave(W, M / ECTA);
     cx<T>* wsp = reinterpret_cast<cx<T>*>(ws);
-    const Plan p = make_plan(m);
     for (long long p0 = 0; p0 < batch; p0 += W)
     {
         const long long w = (batch - p0) < W ? (batch - p0) : W;
+        const Plan p = product_plan<T>(m, w);
         // 1. first forward pass of both operands: fold + twist in the load
         {
             long long ctas = 0;
@@ -253,11 +291,9 @@ static int negacyclic_mul(const T* a, const T* b, T* c, int n_power, int batch, 
         }
         // 2. last forward pass of both, product, first inverse pass
         {
-            long long ctas = 0;
-            f.geo = pass_geo(p, 1, m, 0, w, &ctas);
             f.ws = wsp;
             f.batch = w;
-            int st = launch_fused<T, false>(f, ctas, s);
+            int st = launch_middle<T>(f, p, m, s);
             if (st) return st;
         }
         // 3. last inverse pass: scale, untwist, unfold into c
@@ -323,11 +359,10 @@ static int cyclic_mul(const cx<T>* a, const cx<T>* b, cx<T>* c, int n_power, int
     else
         W = round_wave(W, M / ECTA);
     cx<T>* wsp = reinterpret_cast<cx<T>*>(ws);
-    const Plan p = make_plan(m);
-    if (p.np != 2) return GPUFFT_ERROR_INVALID_N_POWER;
     for (long long p0 = 0; p0 < batch; p0 += W)
     {
         const long long w = (batch - p0) < W ? (batch - p0) : W;
+        const Plan p = product_plan<T>(m, w);
         {
             long long ctas = 0;
             PassArgs<T> k{};
@@ -344,11 +379,9 @@ static int cyclic_mul(const cx<T>* a, const cx<T>* b, cx<T>* c, int n_power, int
             if (st) return st;
         }
         {
-            long long ctas = 0;
-            f.geo = pass_geo(p, 1, m, 0, w, &ctas);
             f.ws = wsp;
             f.batch = w;
-            int st = launch_fused<T, false>(f, ctas, s);
+            int st = launch_middle<T>(f, p, m, s);
             if (st) return st;
         }
         {
