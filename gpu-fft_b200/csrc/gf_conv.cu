@@ -15,9 +15,10 @@
 //
 //   2N <= 8192:  one kernel per product group (vjp_kernel<L, true>);
 //   otherwise:   strided first forward pass of g, a, b (pass_kernel, IN_VJP3),
-//                contiguous middle pass (vjp_kernel<12, false>), strided last
-//                inverse pass keeping the real parts (pass_kernel, OUT_RE2).
-#include "gf_pass.cuh"
+//                contiguous middle pass (tile_product_kernel, TILE_VJP, from two
+//                2048-point tiles per SM on; vjp_kernel<12, false> below that),
+//                strided last inverse pass keeping the real parts (OUT_RE2).
+#include "gf_tile.cuh"
 
 namespace gfb
 {
@@ -129,8 +130,11 @@ template <int L, bool SINGLE> static int launch_vjp_shape(const VjpArgs& a, long
 static long long vjp_wave(int m, long long batch)
 {
     if (m <= EBITS) return batch;
+    // one launch per phase over as many rows as fit 320 MiB of spectra for the
+    // tile kernel's rings (512 rows of N = 2^14, all kernels of the call: four
+    // waves of 128 with the 4096-point middle pass 368 us, one with the tile kernel 187 us)
     const size_t per = 3 * ((size_t)1 << m) * sizeof(cx<float>);
-    long long w = (long long)((48ull << 20) / per);
+    long long w = (long long)((m - tile::LT <= COL_MAX_L ? 320ull << 20 : 48ull << 20) / per);
     if (w < 1) w = 1;
     return w < batch ? w : batch;
 }
@@ -171,10 +175,16 @@ static int linear_vjp(const float* g, const float* a, const float* b, float* ga,
     if (!ws || ws_bytes < per) return GPUFFT_ERROR_WORKSPACE;
     if ((size_t)W * per > ws_bytes) W = (long long)(ws_bytes / per);
     auto* wsp = reinterpret_cast<cx<float>*>(ws);
-    const Plan p = make_plan(m);
     for (long long p0 = 0; p0 < batch; p0 += W)
     {
         const long long w = (batch - p0) < W ? (batch - p0) : W;
+        Plan p = make_plan(m);
+        const bool tiled = m - tile::LT <= COL_MAX_L && (w << (m - tile::LT)) >= 2LL * sm_count();
+        if (tiled)
+        {
+            p.L[0] = m - tile::LT;
+            p.L[1] = tile::LT;
+        }
         long long ctas = 0;
         PassArgs<float> k{};
         k.geo = pass_geo(p, 0, m, 0, 3 * w, &ctas);
@@ -191,10 +201,26 @@ static int linear_vjp(const float* g, const float* a, const float* b, float* ga,
         int st = launch_pass<float, true>(k, p, 0, ctas, s);
         if (st) return st;
 
-        A.geo = pass_geo(p, 1, m, 0, w, &ctas);
-        A.ws = wsp;
-        A.batch = w;
-        st = launch_vjp_shape<EBITS, false>(A, ctas, s);
+        if (tiled)
+        {
+            // G parked; G conj(B) replaces G, then G conj(A) replaces A
+            TileArgs<float> t{};
+            t.park = wsp;
+            t.in[0] = wsp + 2 * w * M;
+            t.out[0] = wsp;
+            t.in[1] = wsp + w * M;
+            t.out[1] = wsp + w * M;
+            t.roots = A.roots;
+            t.m = m;
+            st = launch_tile_product<float, TILE_VJP>(t, w << (m - tile::LT), s);
+        }
+        else
+        {
+            A.geo = pass_geo(p, 1, m, 0, w, &ctas);
+            A.ws = wsp;
+            A.batch = w;
+            st = launch_vjp_shape<EBITS, false>(A, ctas, s);
+        }
         if (st) return st;
 
         PassArgs<float> q{};

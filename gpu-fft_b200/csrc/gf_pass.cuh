@@ -439,6 +439,36 @@ template <typename T> inline double pass_alg_bytes(const PassArgs<T>& a)
 }
 inline const char* kind_name(int fwd) { return fwd ? "fwd" : "inv"; }
 
+// N points j0 + i step of batch entry b through load variant IK. Linear rows and
+// fold pairs of one launch (IN_VJP3) branch once, not per point: behind a branch
+// each point's loads would wait for the one before.
+template <typename T, int IK, int N>
+__device__ __forceinline__ void load_column(const PassArgs<T>& a, long long b, long long j0, long long step, cx<T> (&x)[N])
+{
+    if constexpr (IK == IN_VJP3)
+    {
+        const RealRows<T> rr = real_rows<T>(a, IK, b);
+        const T* p = rr.re + j0;
+        if (rr.im_off >= 0)
+        {
+#pragma unroll
+            for (int i = 0; i < N; i++) x[i] = mk<T>(ld_stream(p + i * step), ld_stream(p + rr.im_off + i * step));
+        }
+        else
+        {
+#pragma unroll
+            for (int i = 0; i < N; i++) x[i] = mk<T>(ld_stream(p + i * step), T(0));
+        }
+#pragma unroll
+        for (int i = 0; i < N; i++) x[i] = cmul<T>(x[i], ldg<T>(a.twist + j0 + i * step));
+    }
+    else
+    {
+#pragma unroll
+        for (int i = 0; i < N; i++) x[i] = load_elem<T>(a, IK, b, j0 + i * step);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Column form of a strided pass of L <= 4 stages. The pass's closed
 // sub-networks are the columns of each stage-s0 group: elements
@@ -487,8 +517,7 @@ __device__ __forceinline__ void col_pass_body(const PassArgs<T>& a, long long id
         for (int i = 0; i < R; i++) un[i] = ldg<T>(a.twist + j0 + i * C);
     }
     cx<T> x[R];
-#pragma unroll
-    for (int i = 0; i < R; i++) x[i] = load_elem<T>(a, IK, b, j0 + i * C);
+    load_column<T, IK, R>(a, b, j0, C, x);
 #pragma unroll
     for (int k = 0; k < L; k++)
     {
@@ -563,8 +592,7 @@ __device__ __forceinline__ void col_pair_body(const PassArgs<T>& a, long long id
     const long long C = 1LL << lc;
     const long long j0 = (g << (m - s0)) + (r & (C - 1)) + hb * C;
     cx<T> x[H];
-#pragma unroll
-    for (int q = 0; q < H; q++) x[q] = load_elem<T>(a, IK, b, j0 + 2 * q * C);
+    load_column<T, IK, H>(a, b, j0, 2 * C, x);
 #pragma unroll
     for (int k = 0; k < L; k++)
     {

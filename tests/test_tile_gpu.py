@@ -52,3 +52,18 @@ def test_cyclic_tile_rows(gf, dev, n_power, batch, dtype):
     want = torch.fft.ifft(torch.fft.fft(a[:3].to(torch.complex128)) * torch.fft.fft(b[:3].to(torch.complex128)))
     err = torch.linalg.norm(c[:3].to(torch.complex128) - want) / torch.linalg.norm(want)
     assert err.item() < (1e-14 if dtype == torch.complex128 else 2e-6) * n_power
+
+
+@pytest.mark.parametrize("n_power,batch", [(13, 74), (14, 37), (15, 19), (16, 10), (16, 9)])
+def test_vjp_tile_rows(gf, dev, n_power, batch):
+    n = 1 << n_power
+    g = torch.Generator(device=dev).manual_seed(n_power * 100 + batch)
+    up = torch.randn(batch, 2 * n, device=dev, generator=g)
+    a, b = torch.randn(2, batch, n, device=dev, generator=g)
+    ga, gb = gf.linear_mul_vjp(up, a, b)
+    fa, fb = gf.linear_mul_vjp(up[-2:].contiguous(), a[-2:].contiguous(), b[-2:].contiguous())
+    assert torch.equal(ga[-2:], fa) and torch.equal(gb[-2:], fb)
+    G = torch.fft.rfft(up[:2].double(), 4 * n)
+    for got, x in ((ga, b), (gb, a)):
+        want = torch.fft.irfft(G * torch.fft.rfft(x[:2].double(), 4 * n).conj(), 4 * n)[:, :n]
+        assert (torch.linalg.norm(got[:2] - want) / torch.linalg.norm(want)).item() < 2e-5
