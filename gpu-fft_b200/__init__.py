@@ -365,9 +365,11 @@ def split_plan(n_power: int, input_bits: int, non_negative: bool = False, precis
 
 def negacyclic_mul_split(a, b, out=None, input_bits=None, non_negative=None, limbs=None, tables=None,
                          workspace=None, stream=None, return_error=False, precision="f32"):
-    """Exact c = a * b mod (X^N + 1) for (batch, N) int32 tensors, computed with FP32
-    (precision="f32", N <= 2^22) or FP64 (precision="f64", N <= 2^17) transforms on
-    limbs; returns an int64 tensor (and the max pre-rounding error)."""
+    """Exact c = a * b mod (X^N + 1) for (batch, N) int32 tensors from a limb plan for
+    FP32 (precision="f32", N <= 2^22, float tables) or FP64 (precision="f64", N <= 2^17,
+    double tables) transforms; returns an int64 tensor (and the max pre-rounding error).
+    Plans within the error model run on FP64 transforms with b whole where that is
+    faster (include/gpufft_b200.h); the integers are the same."""
     import torch
     batch, n = a.shape
     n_power = n.bit_length() - 1
@@ -409,16 +411,14 @@ def set_f64_middle(r8: int) -> int:
 
 
 def set_split_tile(on: int) -> int:
-    """FP32 split products of rings 2^14..2^16 (up to five limbs) run their
-    contiguous stages in the shared-memory tile kernel (1, the default) or in
-    the chain of pass and group-sum kernels (0); a negative value queries.
-    The integers are the same either way. Returns the previous setting."""
+    """Exact products run on FP64 transforms with one operand whole (1, the
+    default) or as the chain of limb passes (0); a negative value queries. The
+    integers are the same either way. Returns the previous setting."""
     return int(lib().gpufft_set_split_tile(int(on)))
 
 
 def split_wait_timeouts(clear: bool = True) -> int:
-    """Bounded waits of the split tile kernel that ran out since the last clear
-    (each makes its call report an infinite error). Synchronous."""
+    """Bounded waits of the exact product that ran out: its kernels have none (0)."""
     n = ctypes.c_uint()
     check(lib().gpufft_split_wait_timeouts(ctypes.byref(n), int(bool(clear))), "split_wait_timeouts")
     return n.value

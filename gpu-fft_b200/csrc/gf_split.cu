@@ -10,20 +10,10 @@
 
 namespace gfb
 {
-// FP32 split products of rings N = 2^14 .. 2^16 with at most six limbs run
-// their contiguous stages in split_tile_kernel (1, the default) or in the
-// five-kernel chain of pass kernels and split_groups (0). Both give the same
-// integers; set by gpufft_set_split_tile. The tile kernel's bulk copies need a
-// 16-byte aligned workspace, and it needs a tile per SM; others take the chain.
+// Exact products run on FP64 transforms with one operand whole (split_exact; 1,
+// the default) or with both operands cut into the plan's limbs (0). Both give the
+// same integers; set by gpufft_set_split_tile.
 static std::atomic<int> g_split_tile{1};
-
-// The tile kernel runs one persistent CTA per SM; a launch with fewer tiles
-// than SMs (a few products) leaves most of the GPU idle and takes the chain.
-static bool split_tile_ok(int m, int k, long long products)
-{
-    return g_split_tile.load(std::memory_order_relaxed) != 0 && m > EBITS && m - SPLIT_TILE_LT <= SPLIT_COL_MAX &&
-           k <= SPLIT_TILE_MAXK && (products << (m - SPLIT_TILE_LT)) >= (long long)sm_count();
-}
 
 // --------------------------------------------------------------------------
 // host side
@@ -163,12 +153,6 @@ static int split_mul(const int32_t* a, const int32_t* b, int64_t* c, int n_power
         long long hoff = 0; // 2^(w-1) (1 + 2^w + ... + 2^(w(k-2)))
         for (int i = 0; i + 1 < k; i++) hoff += 1LL << (w * i + w - 1);
         A.voff = hoff - A.K;
-        // V = x + voff over the input range (|x| < 2^input_bits, or 0 <= x <
-        // 2^input_bits for non-negative inputs)
-        const long long xlo = non_negative ? 0 : -(1LL << input_bits) + 1, xhi = (1LL << input_bits) - 1;
-        A.dig32 = (xlo + A.voff >= (long long)INT32_MIN && xhi + A.voff <= (long long)INT32_MAX && w * (k - 1) <= 30)
-                      ? 1
-                      : 0;
         unsigned long long S = 0; // sum_{l<k-1} 2^(w l)
         for (int i = 0; i + 1 < k; i++) S += 1ULL << (w * i);
         const unsigned long long K = (unsigned long long)A.K;
@@ -188,6 +172,21 @@ static int split_mul(const int32_t* a, const int32_t* b, int64_t* c, int n_power
     {
         cudaError_t e = cudaMemsetAsync(max_err, 0, sizeof(unsigned), s);
         if (e != cudaSuccess) return set_cuda_error(e);
+    }
+    // a plan within the error model is exact, and so is split_exact; a plan chosen
+    // outside it runs as given, so that its error report is its own
+    if (g_split_tile.load(std::memory_order_relaxed))
+    {
+        double mag = 0;
+        const int B = non_negative ? input_bits - 1 : input_bits;
+        if (B - w * (k - 1) <= w - 1 && predicted_error(n_power, B, w, k, non_negative != 0, &mag, PREC) <= 0.2 &&
+            mag < std::ldexp(1.0, PREC - 3))
+        {
+            const cx<double>* t64 = nullptr;
+            if constexpr (!F32) t64 = tab;
+            const int st = split_exact(a, b, c, m, batch, input_bits, non_negative != 0, w, k, t64, ws, ws_bytes, max_err, s);
+            if (st >= 0) return st;
+        }
     }
     const Plan p = make_plan(m);
     for (long long p0 = 0; p0 < batch; p0 += W)
@@ -220,71 +219,6 @@ static int split_mul(const int32_t* a, const int32_t* b, int64_t* c, int n_power
             }
         }
         long long ctas = 0;
-        if constexpr (F32)
-        {
-            if (split_tile_ok(m, k, wv) && (reinterpret_cast<uintptr_t>(ws) & 15) == 0)
-            {
-                // column kernels for the first / last m - 11 stages around the
-                // tile kernel's eleven contiguous stages of every limb and group
-                const int L0 = m - SPLIT_TILE_LT;
-                A.geo = PassGeo{};
-                A.geo.m = m;
-                int st;
-                if (L0 == SPLIT_COL_MAX)
-                {
-                    // 16-point columns: each column on two lanes (half the registers)
-                    const long long threads = 2 * (2 * wv * (M >> L0));
-                    const unsigned blocks = (unsigned)((threads + SPLIT_COL2_THREADS - 1) / SPLIT_COL2_THREADS);
-                    GF_TRACE(tr, (double)wv * M * (2 * 2 * 4 + 2 * k * sizeof(cx<T>)), s,
-                             "split_fwd0_col2<f32,L%d,k%d>", L0, k);
-                    st = dispatch_int<1, SPLIT_TILE_MAXK>(k, [&]<int KK>() {
-                        return A.dig32 ? launch_k(split_fwd0_col2<SPLIT_COL_MAX, KK, true>, blocks,
-                                                  SPLIT_COL2_THREADS, 0, s, A)
-                                       : launch_k(split_fwd0_col2<SPLIT_COL_MAX, KK, false>, blocks,
-                                                  SPLIT_COL2_THREADS, 0, s, A);
-                    });
-                }
-                else
-                {
-                    const long long threads = 2 * wv * (M >> L0);
-                    const unsigned blocks = (unsigned)((threads + SPLIT_COL_THREADS - 1) / SPLIT_COL_THREADS);
-                    GF_TRACE(tr, (double)wv * M * (2 * 2 * 4 + 2 * k * sizeof(cx<T>)), s,
-                             "split_fwd0_col<f32,L%d,k%d>", L0, k);
-                    st = dispatch_int<1, SPLIT_COL_MAX - 1>(L0, [&]<int LL>() {
-                        return dispatch_int<1, SPLIT_TILE_MAXK>(k, [&]<int KK>() {
-                            return launch_k(split_fwd0_col<T, LL, KK>, blocks, SPLIT_COL_THREADS, 0, s, A);
-                        });
-                    });
-                }
-                if (st) return st;
-                st = launch_split_tile(k, A, wv * (M >> SPLIT_TILE_LT), s);
-                if (st) return st;
-                if (L0 == SPLIT_COL_MAX)
-                {
-                    const long long threads = 2 * (wv * (M >> L0));
-                    const unsigned blocks = (unsigned)((threads + SPLIT_COL2_THREADS - 1) / SPLIT_COL2_THREADS);
-                    GF_TRACE(tr, (double)wv * M * ((2 * k - 1) * sizeof(cx<T>) + 2 * 8), s,
-                             "split_inv0_col2<f32,L%d,k%d>", L0, k);
-                    st = dispatch_int<1, SPLIT_TILE_MAXK>(k, [&]<int KK>() {
-                        return launch_k(split_inv0_col2<SPLIT_COL_MAX, KK>, blocks, SPLIT_COL2_THREADS, 0, s, A);
-                    });
-                }
-                else
-                {
-                    const long long threads = wv * (M >> L0);
-                    const unsigned blocks = (unsigned)((threads + SPLIT_COL_THREADS - 1) / SPLIT_COL_THREADS);
-                    GF_TRACE(tr, (double)wv * M * ((2 * k - 1) * sizeof(cx<T>) + 2 * 8), s,
-                             "split_inv0_col<f32,L%d,k%d>", L0, k);
-                    st = dispatch_int<1, SPLIT_COL_MAX - 1>(L0, [&]<int LL>() {
-                        return dispatch_int<1, SPLIT_TILE_MAXK>(k, [&]<int KK>() {
-                            return launch_k(split_inv0_col<T, LL, KK>, blocks, SPLIT_COL_THREADS, 0, s, A);
-                        });
-                    });
-                }
-                if (st) return st;
-                continue;
-            }
-        }
         // rings with one pass (FP64, and FP32 batches too small to fill the
         // SMs) run a zero-stage column form (digits, fold, twist) around that
         // single contiguous pass

@@ -75,7 +75,6 @@ template <typename T> struct SplitArgsT
     int uq, ur;        // K = 2^(w uq + ur): centring term joins groups s = l + uq, scaled 2^ur
     T scale;
     int w, k;
-    int dig32; // every V = x + voff fits an int32 and w (k - 1) <= 30: 32-bit digits
     long long W; // products per wave (stride of the workspace)
     long long batch;
     PassGeo geo;
@@ -402,9 +401,6 @@ template <int L> __global__ void __launch_bounds__(NTHR) split_inv0(const SplitA
 // identical.
 // --------------------------------------------------------------------------
 constexpr int SPLIT_COL_MAX = 4;
-// log2 of the tile kernel's tile (gf_split_tile.cuh); its column passes run the
-// first / last m - SPLIT_TILE_LT stages
-constexpr int SPLIT_TILE_LT = 11;
 constexpr int SPLIT_COL_THREADS = 128;
 
 // One thread per column of one operand of one product: the column's 2 x 2^L0
@@ -472,290 +468,6 @@ __global__ void __launch_bounds__(SPLIT_COL_THREADS) split_fwd0_col(const SplitA
 #pragma unroll
         for (int i = 0; i < R; i++) d[i * C] = x[i];
     }
-}
-
-// Paired-lane column kernels for 2^L0-point columns (L0 >= 2): lanes l and
-// l ^ 16 of a warp share 16 columns, lane half hb = (l >> 4) & 1 holding rows
-// i = 2 m + hb (m < 2^(L0-1)). Every stage with span h >= 2 pairs rows of one
-// parity and runs in the thread (twiddle table[i >> (L0 - s)] = table[m >>
-// (L0 - s - 1)]); the span-1 stage pairs rows 2m and 2m+1 across the two
-// lanes through one register exchange (__shfl_xor_sync). Same butterflies,
-// twiddles and order as split_fwd0_col / split_inv0_col, so the same values, at
-// half the registers per thread.
-constexpr int SPLIT_COL2_THREADS = 128; // five CTAs per SM (forward), four (inverse)
-
-__device__ __forceinline__ void prefetch_l2(const void* p)
-{
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
-__device__ __forceinline__ cx<float> shfl16(cx<float> v)
-{
-    return mk<float>(__shfl_xor_sync(0xffffffffu, v.x, 16), __shfl_xor_sync(0xffffffffu, v.y, 16));
-}
-
-// The float value of a w-bit digit u (< 2^23) minus 2^(w-1): u placed in the
-// mantissa of 2^23, then one exact subtraction.
-__device__ __forceinline__ float digit_f(unsigned u, float bias) { return __int_as_float((int)(u | 0x4B000000u)) - bias; }
-
-// D32: every V = x + voff fits an int32 (a.dig32), digits in 32-bit arithmetic
-template <int L0, int K, bool D32>
-__global__ void __launch_bounds__(SPLIT_COL2_THREADS, 4) split_fwd0_col2(const SplitArgs a)
-{
-    pdl_begin(); // before any global-memory access (programmatic launch)
-    constexpr int R = 1 << L0, H = R / 2;
-    // the tile path's column passes only: m = L0 + SPLIT_TILE_LT, all
-    // column offsets compile-time
-    constexpr int m = L0 + SPLIT_TILE_LT;
-    constexpr long long M = 1LL << m, C = M >> L0;
-    const long long idx = (long long)blockIdx.x * SPLIT_COL2_THREADS + threadIdx.x;
-    const int hb = (int)((idx >> 4) & 1);
-    const long long col = ((idx >> 5) << 4) + (idx & 15); // column over all (operand, product)
-    const long long c = col & (C - 1);
-    const long long bb = col >> (m - L0);
-    const bool ok = bb < 2 * a.W; // the grid covers whole warps; every lane joins the exchange
-    const long long op = bb >= a.W ? 1 : 0, p = ok ? bb - op * a.W : 0;
-    const int32_t* src = (op == 0 ? a.a : a.b) + p * 2 * M + c;
-    using V = typename std::conditional<D32, int, long long>::type;
-    V v0[H], v1[H];
-    cx<float> tw[H];
-#pragma unroll
-    for (int q = 0; q < H; q++)
-    {
-        const long long i = 2 * q + hb;
-        // out-of-range lanes read product 0 (p = 0 keeps src inside the inputs):
-        // their results are never stored, and their exchange partner (lane ^ 16,
-        // the same column) is out of range too
-        v0[q] = (V)((long long)__ldg(src + i * C) + a.voff);
-        v1[q] = (V)((long long)__ldg(src + i * C + M) + a.voff);
-        tw[q] = ldg<float>(a.twist + c + i * C);
-    }
-    // the column's twiddles, the same for every limb: table[0 .. H/2) for the
-    // spans >= 2 and, for the span-1 stage, table[q] on half 1 (half 0 sends
-    // U unchanged, through a multiplication by 1)
-    cx<float> tws[H / 2], t1[H];
-    const float sg = hb ? -1.f : 1.f;
-#pragma unroll
-    for (int q = 0; q < H; q++)
-    {
-        const cx<float> t = ldg<float>(a.roots + q);
-        if (q < H / 2) tws[q] = t;
-        t1[q] = hb ? t : mk<float>(1.f, 0.f);
-    }
-    const int w = a.w;
-    const long long mask = (1LL << w) - 1;
-    const int half = 1 << (w - 1);
-    const float bias = 8388608.f + (float)half; // 2^23 + 2^(w-1)
-    cx<float>* dst = a.spec + (op * K * a.W + p) * M + c;
-#pragma unroll
-    for (int l = 0; l < K; l++)
-    {
-        cx<float> x[H];
-#pragma unroll
-        for (int q = 0; q < H; q++)
-        {
-            float f0, f1;
-            if constexpr (D32)
-            {
-                // 32-bit digits: extract, then convert through the mantissa
-                if (l < K - 1)
-                {
-                    f0 = digit_f(((unsigned)v0[q] >> (w * l)) & (unsigned)mask, bias);
-                    f1 = digit_f(((unsigned)v1[q] >> (w * l)) & (unsigned)mask, bias);
-                }
-                else
-                {
-                    f0 = (float)(v0[q] >> (w * l));
-                    f1 = (float)(v1[q] >> (w * l));
-                }
-            }
-            else
-            {
-                int d0, d1;
-                if (l < K - 1)
-                {
-                    d0 = (int)(v0[q] & mask) - half;
-                    d1 = (int)(v1[q] & mask) - half;
-                    v0[q] >>= w;
-                    v1[q] >>= w;
-                }
-                else
-                {
-                    d0 = (int)v0[q];
-                    d1 = (int)v1[q];
-                }
-                f0 = (float)d0;
-                f1 = (float)d1;
-            }
-            x[q] = cmul<float>(mk<float>(f0, f1), tw[q]);
-        }
-        // stages s = 0 .. L0-2 (span h = 2^(L0-1-s) >= 2): rows q and q + h/2 of this lane
-#pragma unroll
-        for (int s = 0; s < L0 - 1; s++)
-        {
-            const int hh = 1 << (L0 - 2 - s);
-#pragma unroll
-            for (int q = 0; q < H; q++)
-                if (!(q & hh)) ct_bfly<float>(x[q], x[q + hh], tws[q >> (L0 - 1 - s)]);
-        }
-        // stage L0-1 (span 1): U = row 2q (half 0), V = row 2q+1 (half 1),
-        // table[q]: half 1 sends V table[q], half 0 sends U; half 0 keeps the
-        // sum, half 1 the difference
-#pragma unroll
-        for (int q = 0; q < H; q++)
-        {
-            const cx<float> mine = cmul<float>(x[q], t1[q]);
-            const cx<float> other = shfl16(mine);
-            x[q] = __ffma2_rn(mine, make_float2(sg, sg), other);
-        }
-        if (ok)
-        {
-            cx<float>* d = dst + (long long)l * a.W * M;
-#pragma unroll
-            for (int q = 0; q < H; q++) d[(2 * q + hb) * C] = x[q];
-        }
-    }
-}
-
-// Round-to-nearest-even of |v| < 2^22 by one addition: v + 1.5 2^23 lands in
-// [2^23, 2^24), where the float spacing is 1, and the integer is the low bits
-// of the sum's encoding. Larger values are not certified (group_error), so
-// their integer does not matter.
-constexpr float RND_MAGIC = 12582912.0f; // 1.5 * 2^23
-constexpr int RND_MAGIC_BITS = 0x4B400000;
-
-// acc + i 2^sh (mod 2^64) in the form MODE names (the caller picks it once
-// per group, sh being uniform): 0 one wide multiply-add (sh <= 30), 1 one add
-// to the high word (sh >= 32), 2 a 64-bit shift (sh = 31)
-template <int MODE> __device__ __forceinline__ long long add_shifted(long long acc, int i, int sh)
-{
-    if constexpr (MODE == 0) return acc + (long long)i * (long long)(1 << sh);
-    if constexpr (MODE == 1)
-        return (long long)((unsigned long long)acc + ((unsigned long long)((unsigned)i << (sh - 32)) << 32));
-    return (long long)((unsigned long long)acc + ((unsigned long long)(long long)i << sh));
-}
-
-template <int L0, int K> __global__ void __launch_bounds__(SPLIT_COL2_THREADS, 4) split_inv0_col2(const SplitArgs a)
-{
-    pdl_begin(); // before any global-memory access (programmatic launch)
-    constexpr int R = 1 << L0, H = R / 2;
-    // the tile path's column passes only: m = L0 + SPLIT_TILE_LT, all
-    // column offsets compile-time
-    constexpr int m = L0 + SPLIT_TILE_LT;
-    constexpr long long M = 1LL << m, C = M >> L0;
-    const long long idx = (long long)blockIdx.x * SPLIT_COL2_THREADS + threadIdx.x;
-    const int hb = (int)((idx >> 4) & 1);
-    const long long col = ((idx >> 5) << 4) + (idx & 15);
-    const long long c = col & (C - 1);
-    const long long p0 = col >> (m - L0);
-    const bool ok = p0 < a.W;
-    const long long p = ok ? p0 : 0;
-    cx<float> un[H];
-#pragma unroll
-    for (int q = 0; q < H; q++)
-    {
-        const cx<float> u = ldg<float>(a.untwist + c + (2 * q + hb) * C);
-        un[q] = mk<float>(u.x * a.scale, u.y * a.scale); // scale folded in: exact, scale is 2^-m
-    }
-    // the column's twiddles, the same for every group: table[0 .. H) for the
-    // span-1 stage (half 1 multiplies its difference; half 0 passes its sum on
-    // through a multiplication by 1) and table[0 .. H/2) for the others
-    cx<float> t1[H], tw[H / 2];
-    const float sg = hb ? -1.f : 1.f;
-#pragma unroll
-    for (int q = 0; q < H; q++)
-    {
-        const cx<float> t = ldg<float>(a.inv_roots + q);
-        if (q < H / 2) tw[q] = t;
-        t1[q] = hb ? t : mk<float>(1.f, 0.f);
-    }
-    long long acc_lo[H], acc_hi[H];
-#pragma unroll
-    for (int q = 0; q < H; q++) acc_lo[q] = acc_hi[q] = 0;
-    float err = 0.f, big = 0.f;
-    const cx<float>* src = a.group + p * M + c + hb * C;
-    const long long gstride = a.W * M;
-    cx<float> nx[H];
-#pragma unroll
-    for (int q = 0; q < H; q++) nx[q] = __ldcs(src + 2 * q * C);
-    // group s + 1 is loaded into registers while group s is transformed, and
-    // group s + 2 is prefetched into L2 (more bytes in flight than the
-    // registers could hold)
-    if (2 * K - 1 > 1)
-    {
-#pragma unroll
-        for (int q = 0; q < H; q++) prefetch_l2(src + gstride + 2 * q * C);
-    }
-#pragma unroll 1
-    for (int s = 0; s < 2 * K - 1; s++)
-    {
-        cx<float> x[H];
-#pragma unroll
-        for (int q = 0; q < H; q++) x[q] = nx[q];
-        if (s + 2 < 2 * K - 1)
-        {
-#pragma unroll
-            for (int q = 0; q < H; q++) prefetch_l2(src + (s + 2) * gstride + 2 * q * C);
-        }
-        if (s + 1 < 2 * K - 1)
-        {
-#pragma unroll
-            for (int q = 0; q < H; q++) nx[q] = __ldcs(src + (s + 1) * gstride + 2 * q * C);
-        }
-        // stage L0-1 (span 1) first: U = row 2q (half 0), V = row 2q+1 (half 1),
-        // table[q]: half 0 keeps U + V, half 1 takes (U - V) table[q]
-#pragma unroll
-        for (int q = 0; q < H; q++)
-        {
-            const cx<float> other = shfl16(x[q]);
-            x[q] = cmul<float>(__ffma2_rn(x[q], make_float2(sg, sg), other), t1[q]);
-        }
-        // stages L0-2 .. 0 (span 2^(L0-1-st) >= 2), rows q and q + h/2 of this lane
-#pragma unroll
-        for (int st = L0 - 2; st >= 0; st--)
-        {
-            const int hh = 1 << (L0 - 2 - st);
-#pragma unroll
-            for (int q = 0; q < H; q++)
-                if (!(q & hh)) gs_bfly<float>(x[q], x[q + hh], tw[q >> (L0 - 1 - st)]);
-        }
-        const int sh = a.w * s;
-        auto finish = [&](auto mode) {
-            constexpr int MODE = decltype(mode)::value;
-#pragma unroll
-            for (int q = 0; q < H; q++)
-            {
-                const cx<float> v = cmul<float>(x[q], un[q]);
-                const float tr = __fadd_rn(v.x, RND_MAGIC), ti = __fadd_rn(v.y, RND_MAGIC);
-                err = fmaxf(err, fmaxf(fabsf(__fsub_rn(v.x, __fsub_rn(tr, RND_MAGIC))),
-                                       fabsf(__fsub_rn(v.y, __fsub_rn(ti, RND_MAGIC)))));
-                big = fmaxf(big, fmaxf(fabsf(v.x), fabsf(v.y)));
-                acc_lo[q] = add_shifted<MODE>(acc_lo[q], __float_as_int(tr) - RND_MAGIC_BITS, sh);
-                acc_hi[q] = add_shifted<MODE>(acc_hi[q], __float_as_int(ti) - RND_MAGIC_BITS, sh);
-            }
-        };
-        // one uniform branch per group
-        if (sh <= 30)
-            finish(std::integral_constant<int, 0>{});
-        else if (sh >= 32)
-            finish(std::integral_constant<int, 1>{});
-        else
-            finish(std::integral_constant<int, 2>{});
-    }
-    if (ok)
-    {
-        int64_t* dst = a.c + p * 2 * M + c;
-#pragma unroll
-        for (int q = 0; q < H; q++)
-        {
-            const long long i = 2 * q + hb;
-            const long long j = c + i * C;
-            __stcs(reinterpret_cast<long long*>(dst + i * C), acc_lo[q] + uu_term(a, j, 2 * M));
-            __stcs(reinterpret_cast<long long*>(dst + i * C + M), acc_hi[q] + uu_term(a, j + M, 2 * M));
-        }
-    }
-    // values of 2^22 or more are not certified (group_error)
-    report_err(a.max_err, ok ? (big >= 4194304.0f ? 1.0f : err) : 0.f);
 }
 
 // FP32 columns of 8 points fit 128 registers: four CTAs (16 warps) per
@@ -913,12 +625,12 @@ template <int L, bool SINGLE, int K> static int launch_mid_k(const SplitArgs& a,
     return launch_split(split_mid<L, SINGLE, K>, done, a, ctas, s);
 }
 
-// The split product's contiguous stages of every limb and limb group on
-// 2^SPLIT_TILE_LT-point tiles held in shared memory (gf_split_tile.cuh), for
-// up to SPLIT_TILE_MAXK limbs; compiled in gf_split_tile.cu.
-// (SPLIT_TILE_LT is defined with the column kernels above.)
-constexpr int SPLIT_TILE_MAXK = 5;
-int launch_split_tile(int k, const SplitArgs& a, long long tiles, cudaStream_t s);
+// The exact product on FP64 transforms (gf_split_tile.cuh), or -1 where it does
+// not apply (the caller then runs the limb plan): tables is the FP64 native block,
+// or null (FP32 callers): the call then makes its own twiddles in the workspace.
+// (plan_w, plan_k): the caller's limb plan, whose exactness is kept.
+int split_exact(const int32_t* a, const int32_t* b, int64_t* c, int m, int batch, int input_bits, bool non_negative,
+                int plan_w, int plan_k, const cx<double>* tables, void* ws, size_t ws_bytes, unsigned* max_err, cudaStream_t s);
 
 // one-kernel products for rings N <= 8192 (transform length 2^L, L = 1..12),
 // compiled in separate translation units by L range

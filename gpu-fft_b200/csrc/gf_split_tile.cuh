@@ -1,513 +1,456 @@
-// gpufft-b200: the split product's middle on 2048-point tiles held in shared
-// memory (rings N = 2^14 .. 2^16, up to six limbs).
+// gpufft-b200: the exact (split) product on FP64 transforms, with one operand cut
+// into limbs and the other whole.
 //
-// The split product (gf_split.cuh) transforms 2k limb polynomials, forms 2k-1
-// limb-group sums per spectral point and inverse-transforms every group. Each
-// transform of M = N/2 points has m = log2 M stages; the first L0 = m - 11 run
-// in the column kernels (split_fwd0_col / split_inv0_col), the other eleven on
-// contiguous tiles of 2048 points. This kernel runs, for one tile of one
-// product, every one of those contiguous stages of all 2k limbs, the group
-// sums and the contiguous stages of all 2k-1 groups without leaving the SM:
+// c = a b mod (X^N + 1) for integers |a_i|, |b_i| < 2^B. An FP64 transform pair
+// leaves an error of about 7 rms(a) rms(b) sqrt(N log2 N) 2^-53 per coefficient
+// (the model of gf_split.cu): at B = 23 and N = 2^16 that is 18, far above 0.5, but
+// with a alone cut into K = 2 limbs of 12 bits it is 0.005. So a is cut into the
+// fewest limbs (one up to about 18 bits, two at 24) and b stays whole: K + 1
+// forward and K inverse FP64 transforms, where equal FP32 limbs of both operands
+// take 4k - 1 (19 for 24 bits) and equal FP64 limbs 4K - 1. B200 runs FP64 at half
+// the FP32 rate, so 5 against 19 is a quarter of the arithmetic, and the spectra
+// in memory fall from 19 x 8 to 3 x 16 bytes per point. The integers are the same.
 //
-//   slots       2k shared-memory slots of one tile (16 KB each, 160 KB for
-//               k = 5, 192 KB for k = 6); limb tile tau is bulk-copied (cp.async.bulk, the TMA
-//               unit) from the column kernel's output into slot tau, completed
-//               on mbarrier tau;
-//   teams       the CTA's 512 threads are four teams of 128 (16 points per
-//               thread); a team transforms one limb or group at a time, in
-//               place in its slot: eleven stages as three radix-16 register
-//               rounds (e-bits [7,11), [3,7), [0,3)) with the slot itself as
-//               the transpose buffer, point e at the padded position
-//               e + (e >> 4), where every register window is free of bank
-//               conflicts and every register's address is a per-thread base
-//               plus a compile-time offset (the bulk copy lands unpadded in
-//               the slot's first 16 KB, read once by the first round);
-//   groups      all 512 threads form G_s = sum_{i+j=s} A_i B_j (+ the centring
-//               term) at every point and write G_s over slot s;
-//   queue       the CTA is persistent; the inverse items of tile i (the eleven
-//               stages of each group in the reverse order, then the group tile
-//               to the workspace for split_inv0_col) and the forward items of
-//               tile i+1 share one work queue that the teams draw from, so
-//               the teams stay busy across the tile boundary; each inverse item
-//               starts the bulk copy of the next tile's limb into its slot as
-//               soon as its team has read the slot, so loads overlap compute.
+// Non-negative inputs are centred, a = a' + C u, b = b' + C u (C = 2^B, u the
+// all-ones polynomial):
+//     a b = sum_l 2^(w l) A_l (b' + C u) + C u b' + C^2 u u.
+// The tile kernel forms A_l (B' + C U), adds 2^(B - w(K-1)) U B' to the last limb's
+// product (U = transform of u), and C^2 u u is added exactly in int64.
 //
-// HBM traffic per product drops from the five-kernel chain's four passes over
-// the limb and group spectra to two (the column kernels' write and read stay).
-// Butterflies and twiddle indices are the engine's (table[(T << u) + (e >>
-// (11 - u))] at stage L0 + u for tile T), so the spectra equal the engine
-// path's up to the order of floating-point operations inside a round.
+// Kernels, rings N = 2^14 .. 2^17 (transforms of 2^m points, m = N's log2 - 1):
+//   exact_fwd_col   digits, fold, twist and the first m - 11 stages of every limb
+//                   of a and of b (a column of 2^(m-11) points on one lane, on two
+//                   from 16 points on);
+//   exact_tile      the eleven stages on 2048-point tiles of b (parked in
+//                   registers) and of each limb, the product, the inverse stages
+//                   (gf_tile.cuh);
+//   exact_inv_col   last inverse stages, rounding, the error report and the int64
+//                   sum of the limbs' products.
+// Rings N = 2^5 .. 2^13 run in one kernel, exact_single, a CTA holding whole
+// products.
 //
-// Waits on the mbarriers are bounded (gf_async.cuh). A team whose wait runs out
-// reports it at the next CTA-wide barrier; the CTA then marks the call's error
-// report as infinite (not exact), counts the timeout in g_split_wait_timeouts,
-// drains its outstanding copies with a bounded wait and returns.
+// Measured (B200): N = 2^16, batch 256, 24 bits: 413 us (columns 109 + 85, tiles
+// 222, tables 3) where five FP32 limbs of both operands on shared-memory tiles took
+// 824; N = 2^13, batch 333, 16 bits: 40 us against 360; N = 2^12, batch 2000, 16
+// bits: 87 against 809; one product of N = 2^12: 19 against 24.
 #pragma once
 
-#include <type_traits>
-
-#include "gf_async.cuh"
 #include "gf_split.cuh"
+#include "gf_tile.cuh"
 
 namespace gfb
 {
-namespace stile
-{
-constexpr int LT = SPLIT_TILE_LT; // log2 points per tile (11)
-constexpr int P = 1 << LT; // 2048 points per tile
-constexpr int HT = 128;    // threads per team
-constexpr int R = P / HT;  // 16 points per thread
-constexpr int MAXK = SPLIT_TILE_MAXK; // limb counts whose 2k slots fit in shared memory (5: 10 slots, 170 KB)
-constexpr int SLOT = P + P / 16;      // padded slot (2176 points, 17 KB)
 
-// e of register 0 of thread t (0..127) when the registers are the four e-bits
-// [W, W+4): the thread supplies the other seven bits in order
-template <int W> __device__ __forceinline__ int ebase(int t)
-{
-    return (t & ((1 << W) - 1)) | ((t >> W) << (W + 4));
-}
-__device__ __forceinline__ constexpr int ppos(int e) { return e + (e >> 4); }
+constexpr int EXACT_MAX_LIMBS = 3;
 
-// Padded slot addresses of a thread's 16 registers in window W:
-// ppos(ebase(t) + (r << W)) = ppos(ebase(t)) + off(r), because the window bits
-// of ebase are clear and no addition carries across bit 4:
-//   W = 7: off = 136 r;  W = 3: off = 8 r + (r >> 1);  W = 0: off = r.
-template <int W> struct SlotAddr
+struct ExactArgs
 {
-    int b;
-    __device__ __forceinline__ explicit SlotAddr(int t) : b(ppos(ebase<W>(t))) {}
-    __device__ __forceinline__ int operator()(int r) const { return b + (r << W) + ((r << W) >> 4); }
+    const int32_t* a;
+    const int32_t* b;
+    int64_t* c;
+    cx<double>* spec; // [K+1][W][M]: a's limbs, then b
+    const cx<double>* roots;
+    const cx<double>* twist;
+    const cx<double>* uspec; // U; each 4096-point tile permuted e -> (e >> 4) + 256 (e & 15) when M > 4096
+    unsigned* max_err;       // float bits of the largest pre-rounding error (may be null)
+    long long cen;           // centring offset C (0: none)
+    long long voff;          // digits of a: V = x + voff
+    double ushift;           // 2^(B - w(K-1)): weight of U B' in the last limb's product
+    double scale;
+    int w;       // limb width
+    long long W; // products of this launch
 };
 
-// Window-0 twiddles of a tile (stages u = 8, 9, 10 on e-bits 2, 1, 0): thread
-// t's are table[(T << u) + (16 t >> (11 - u)) + h] for h < 2^(u - 7), i.e.
-// pairs (T << (u - 1)) + 2^(u - 8) t + i for i < 2^(u - 8): one pair at u = 8,
-// two at u = 9, four at u = 10 -- seven 16-byte pairs, 1792 entries per tile.
-// Read straight from the table, a warp's paired loads would stride 64 bytes
-// (half of every sector wasted, sixteen cache lines per instruction); staged
-// thread-major in shared memory (pair j of thread t at j * 128 + t) each round
-// reads them conflict-free. w0_pair(pb) is the first pair index j of the
-// stage on e-bit pb.
-__device__ __forceinline__ constexpr int w0_pair(int pb) { return pb == 2 ? 0 : (pb == 1 ? 1 : 3); }
-constexpr int W0_PAIRS = 7 * HT; // float4 per staged table
-
-// All 512 threads copy the window-0 twiddles of tile T (table `tw`, 16-byte
-// aligned when `vec`) into `dst` (W0_PAIRS float4).
-__device__ __forceinline__ void stage_w0(float4* dst, const cx<float>* __restrict__ tw, long long T, int tid,
-                                         int nthreads, bool vec)
+// The pointer again, hidden from the compiler: table entries used by several
+// limbs are loaded for each (they are in L1) instead of being kept in registers.
+__device__ __forceinline__ const cx<double>* fresh(const cx<double>* p)
 {
-    // linear pair p over the three stages: [0, 128) u = 8, [128, 384) u = 9, [384, 896) u = 10
-    for (int p = tid; p < W0_PAIRS; p += nthreads)
-    {
-        int u, q, t, j;
-        if (p < 128)
-        {
-            u = 8, q = p, t = q, j = 0;
-        }
-        else if (p < 384)
-        {
-            u = 9, q = p - 128, t = q >> 1, j = 1 + (q & 1);
-        }
-        else
-        {
-            u = 10, q = p - 384, t = q >> 2, j = 3 + (q & 3);
-        }
-        const cx<float>* src = tw + (T << u) + 2 * q;
-        float4 v;
-        if (vec)
-        {
-            v = __ldg(reinterpret_cast<const float4*>(src));
-        }
-        else
-        {
-            const cx<float> a = ldg<float>(src), b = ldg<float>(src + 1);
-            v = make_float4(a.x, a.y, b.x, b.y);
-        }
-        dst[j * HT + t] = v;
-    }
+    asm volatile("" : "+l"(p));
+    return p;
 }
 
-// Twiddles of the outer rounds (windows 7 and 3: stages u = 0 .. 7 of the
-// tile) use table[(T << u) + i] for i < 2^u only (window 7: all threads the
-// same 2^u entries; window 3: thread t the 2^(u-4) entries from i = (t >> 3)
-// 2^(u-4)). Staged as entry 2^u + i of a 256-entry buffer, every pair stays
-// 16-byte aligned.
-constexpr int W37_ENTRIES = 256;
+// 1.5 2^52 and its encoding: v + MAGIC is v rounded to the nearest even integer
+// for |v| < 2^51, and the integer is the sum's encoding minus MAGIC's.
+constexpr double RND64 = 6755399441055744.0;
+constexpr long long RND64_BITS = 0x4338000000000000LL;
 
-__device__ __forceinline__ void stage_w37(cx<float>* dst, const cx<float>* __restrict__ tw, long long T, int tid,
-                                          int nthreads)
+// The double value of a 32-bit integer, through the mantissa of 2^52 (one
+// addition instead of a conversion instruction).
+__device__ __forceinline__ double int_f64(int d)
 {
-    for (int idx = tid + 1; idx < W37_ENTRIES; idx += nthreads)
-    {
-        const int u = 31 - __clz(idx);
-        dst[idx] = ldg<float>(tw + (T << u) + (idx - (1 << u)));
-    }
+    return __hiloint2double(0x43300000, d ^ (int)0x80000000) - 4503601774854144.0; // 2^52 + 2^31
 }
 
-// One round: the butterflies of e-bits [LO, HI) inside window W. Stage u of the
-// tile's eleven (e-bit q = 10 - u) pairs e with e + 2^q and uses
-// table[(T << u) + (e >> (q + 1))]; for register r (bit pb of r = q - W clear)
-// that is table[base + (r >> (pb + 1))] with base = (T << u) + (eb >> (q + 1)):
-// 2^(3 - pb) consecutive entries, loaded first so their latencies overlap.
-template <bool FWD, int W, int LO, int HI>
-__device__ __forceinline__ void round(cx<float> (&x)[R], const cx<float>* __restrict__ tw, long long T, int eb,
-                                      bool vec, const float4* staged = nullptr, int t = 0,
-                                      const cx<float>* outer = nullptr)
+// Digit l of K of a's coefficient (balanced; the last takes what is left); K = 1
+// (and b) the centred value itself.
+template <int K> __device__ __forceinline__ int exact_digit(int x, long long voff, int l, int w)
 {
-    constexpr int A = LO - W, RB = HI - LO;
-    static_assert(A >= 0 && RB >= 1 && A + RB <= 4, "the round's bits lie in its window");
-    cx<float> w[15];
+    if (K == 1) return (int)((long long)x + voff);
+    const long long V = (long long)x + voff;
+    if (l == K - 1) return (int)(V >> (w * l));
+    return (int)(((unsigned)(V >> (w * l))) & ((1u << w) - 1)) - (1 << (w - 1));
+}
+
+// Largest distance to the nearest integer and largest magnitude, kept as the high
+// words of the doubles (ordered like the values, 20 bits of mantissa).
+struct ExactErr
+{
+    int e = 0, big = 0;
+    __device__ __forceinline__ void add(double d, double v)
+    {
+        e = max(e, __double2hiint(fabs(d)));
+        big = max(big, __double2hiint(fabs(v)));
+    }
+    // above 2^50 the distance no longer certifies anything (group_error)
+    __device__ __forceinline__ float value() const
+    {
+        if (big >= 0x43100000) return 1.0f;
+        return e == 0 ? 0.f : fminf((float)__hiloint2double(e, -1), 0.5f); // rounded up; a distance is at most 0.5
+    }
+};
+
+// C^2 u u: coefficient j is C^2 (2j + 2 - N)
+__device__ __forceinline__ long long exact_uu(long long cen, long long j, long long N)
+{
+    return (long long)((unsigned long long)cen * (unsigned long long)cen * (unsigned long long)(2 * j + 2 - N));
+}
+
+// ---------------------------------------------------------------------------
+// column kernels: m = L + 11, columns of 2^L points 2048 apart
+// ---------------------------------------------------------------------------
+// One lane per column up to 8 points, two (the rows of one parity each) from 16.
+template <int L> constexpr bool exact_pair() { return L >= 4; }
+template <int L> constexpr int exact_rows() { return exact_pair<L>() ? 1 << (L - 1) : 1 << L; }
+
+// The column's stages on its rows (lane half hb of a pair): the butterflies,
+// twiddles and order of col_pass_kernel. Inverse twiddles are conjugate roots.
+template <bool FWD, int L>
+__device__ __forceinline__ void exact_stages(cx<double> (&x)[exact_rows<L>()], const cx<double>* __restrict__ roots, int hb)
+{
+    constexpr bool PAIR = exact_pair<L>();
+    constexpr int H = exact_rows<L>();
 #pragma unroll
-    for (int k = 0; k < RB; k++)
+    for (int k = 0; k < L; k++)
     {
-        const int pb = FWD ? (A + RB - 1 - k) : (A + k);
-        const int q = W + pb;
-        const int u = LT - 1 - q;
-        const int nt = 1 << (3 - pb);
-        const cx<float>* p0 = tw + (T << u) + (eb >> (q + 1));
-        cx<float>* wk = w + nt - 1;
-        if constexpr (W == 7 || W == 3)
+        const int u = FWD ? k : L - 1 - k;
+        if (PAIR && u == L - 1)
         {
-            if (outer)
+#pragma unroll
+            for (int q = 0; q < H; q++)
             {
-                // entries 2^u + i, i = (eb >> (q + 1)) = 0 (window 7) or (t >> 3) 2^(u-4) (window 3)
-                const cx<float>* q0 = outer + (1 << u) + (eb >> (q + 1));
-                if (nt >= 2)
+                cx<double> wt = ldg<double>(roots + q);
+                if (FWD)
                 {
-#pragma unroll
-                    for (int h = 0; h < nt; h += 2)
-                    {
-                        const float4 v = *reinterpret_cast<const float4*>(q0 + h);
-                        wk[h] = mk<float>(v.x, v.y);
-                        wk[h + 1] = mk<float>(v.z, v.w);
-                    }
+                    const cx<double> mine = hb ? cmul<double>(x[q], wt) : x[q];
+                    const cx<double> other = shfl_half<double>(mine);
+                    x[q] = hb ? csub<double>(other, mine) : cadd<double>(mine, other);
                 }
                 else
                 {
-                    wk[0] = q0[0];
+                    wt.y = -wt.y;
+                    const cx<double> other = shfl_half<double>(x[q]);
+                    x[q] = hb ? cmul<double>(csub<double>(other, x[q]), wt) : cadd<double>(x[q], other);
                 }
-                continue;
+            }
+            continue;
+        }
+        const int lg = (PAIR ? L - 2 : L - 1) - u; // log2 of the pair's distance in rows of this lane
+#pragma unroll
+        for (int q = 0; q < H; q++)
+        {
+            if (q & (1 << lg)) continue;
+            cx<double> wt = ldg<double>(roots + (q >> (lg + 1)));
+            if (FWD)
+            {
+                ct_bfly<double>(x[q], x[q + (1 << lg)], wt);
+            }
+            else
+            {
+                wt.y = -wt.y;
+                gs_bfly<double>(x[q], x[q + (1 << lg)], wt);
             }
         }
-        if constexpr (W == 0 && LO == 0 && HI == 3)
-        {
-            if (staged)
-            {
-                // the tile's window-0 twiddles, staged thread-major (see stage_w0)
+    }
+}
+
+constexpr int EXACT_COL_THREADS = 128;
+
+template <int L, int K>
+__global__ void __launch_bounds__(EXACT_COL_THREADS, L <= 3 ? 6 : 4) exact_fwd_col(const ExactArgs a)
+{
+    pdl_begin(); // before any global-memory access (programmatic launch)
+    constexpr bool PAIR = exact_pair<L>();
+    constexpr int H = exact_rows<L>(), LS = PAIR ? 2 : 1;
+    constexpr long long C = 2048, M = C << L;
+    const long long idx = (long long)blockIdx.x * EXACT_COL_THREADS + threadIdx.x;
+    const int hb = PAIR ? (int)((idx >> 4) & 1) : 0;
+    const long long col = PAIR ? ((idx >> 5) << 4) + (idx & 15) : idx; // over (operand, product, column)
+    const long long c = (col & (C - 1)) + hb * C;
+    const long long bb = col >> 11; // the grid covers whole columns: C is a multiple of the block
+    const bool isb = bb >= a.W;
+    const long long p = isb ? bb - a.W : bb;
+    const int32_t* src = (isb ? a.b : a.a) + p * 2 * M + c;
+    int v0[H], v1[H];
 #pragma unroll
-                for (int h = 0; h < nt; h += 2)
-                {
-                    const float4 v = staged[(w0_pair(pb) + (h >> 1)) * HT + t];
-                    wk[h] = mk<float>(v.x, v.y);
-                    wk[h + 1] = mk<float>(v.z, v.w);
-                }
-                continue;
-            }
+    for (int q = 0; q < H; q++)
+    {
+        v0[q] = __ldg(src + q * LS * C);
+        v1[q] = __ldg(src + q * LS * C + M);
+    }
+    auto transform = [&](auto digit, cx<double>* dst) {
+        cx<double> x[H];
+        const cx<double>* tw = fresh(a.twist) + c;
+#pragma unroll
+        for (int q = 0; q < H; q++)
+            x[q] = cmul<double>(mk<double>(int_f64(digit(v0[q])), int_f64(digit(v1[q]))), ldg<double>(tw + q * LS * C));
+        exact_stages<true, L>(x, fresh(a.roots), hb);
+#pragma unroll
+        for (int q = 0; q < H; q++) dst[q * LS * C] = x[q];
+    };
+    cx<double>* dst = a.spec + p * M + c;
+    if (isb)
+    {
+        transform([&](int x) { return (int)((long long)x - a.cen); }, dst + K * a.W * M);
+        return;
+    }
+#pragma unroll 1
+    for (int l = 0; l < K; l++)
+    {
+        long long voff = a.voff;
+        asm volatile("" : "+l"(voff)); // x + voff is formed per limb, not kept in registers
+        transform([&](int x) { return exact_digit<K>(x, voff, l, a.w); }, dst + l * a.W * M);
+    }
+}
+
+template <int L, int K>
+__global__ void __launch_bounds__(EXACT_COL_THREADS, L == 5 ? 2 : K > 1 ? 4 : 5) exact_inv_col(const ExactArgs a)
+{
+    pdl_begin(); // before any global-memory access (programmatic launch)
+    constexpr bool PAIR = exact_pair<L>();
+    constexpr int H = exact_rows<L>(), LS = PAIR ? 2 : 1;
+    constexpr long long C = 2048, M = C << L;
+    const long long idx = (long long)blockIdx.x * EXACT_COL_THREADS + threadIdx.x;
+    const int hb = PAIR ? (int)((idx >> 4) & 1) : 0;
+    const long long col = PAIR ? ((idx >> 5) << 4) + (idx & 15) : idx;
+    const long long c = (col & (C - 1)) + hb * C;
+    const long long p = col >> 11;
+    const cx<double>* src = a.spec + p * M + c;
+    long long lo[H], hi[H];
+#pragma unroll
+    for (int q = 0; q < H; q++)
+    {
+        const long long j = c + q * LS * C;
+        lo[q] = exact_uu(a.cen, j, 2 * M);
+        hi[q] = exact_uu(a.cen, j + M, 2 * M);
+    }
+    ExactErr err;
+    // the next limb's loads are in flight while this one is transformed
+    cx<double> nx[H];
+#pragma unroll
+    for (int q = 0; q < H; q++) nx[q] = __ldcs(src + q * LS * C);
+#pragma unroll 1
+    for (int l = 0; l < K; l++)
+    {
+        cx<double> x[H];
+#pragma unroll
+        for (int q = 0; q < H; q++) x[q] = nx[q];
+        if (l + 1 < K)
+        {
+#pragma unroll
+            for (int q = 0; q < H; q++) nx[q] = __ldcs(src + (l + 1) * a.W * M + q * LS * C);
         }
-        if (nt >= 2 && vec)
+        exact_stages<false, L>(x, fresh(a.roots), hb);
+        const cx<double>* tw = fresh(a.twist) + c;
+        const int sh = a.w * l;
+#pragma unroll
+        for (int q = 0; q < H; q++)
+        {
+            const cx<double> t = ldg<double>(tw + q * LS * C);
+            // untwist = conj(twist); the scale is a power of two
+            const cx<double> v = cmul<double>(x[q], mk<double>(t.x * a.scale, -t.y * a.scale));
+            const double r0 = __dadd_rn(v.x, RND64), r1 = __dadd_rn(v.y, RND64);
+            err.add(__dsub_rn(v.x, __dsub_rn(r0, RND64)), v.x);
+            err.add(__dsub_rn(v.y, __dsub_rn(r1, RND64)), v.y);
+            const long long i0 = __double_as_longlong(r0) - RND64_BITS, i1 = __double_as_longlong(r1) - RND64_BITS;
+            lo[q] = (long long)((unsigned long long)lo[q] + ((unsigned long long)i0 << sh));
+            hi[q] = (long long)((unsigned long long)hi[q] + ((unsigned long long)i1 << sh));
+        }
+    }
+    long long* dst = reinterpret_cast<long long*>(a.c + p * 2 * M + c);
+#pragma unroll
+    for (int q = 0; q < H; q++)
+    {
+        __stcs(dst + q * LS * C, lo[q]);
+        __stcs(dst + q * LS * C + M, hi[q]);
+    }
+    report_err(a.max_err, err.value());
+}
+
+// The product of a limb's spectrum value x with b's (pk); `last`: the limb that U B'
+// joins.
+__device__ __forceinline__ cx<double> exact_product(cx<double> x, cx<double> pk, const ExactArgs& a, double ui, bool last)
+{
+    // U = 1 + i ui
+    const double C = (double)a.cen;
+    cx<double> v = cmul<double>(x, mk<double>(pk.x + C, rfma(C, ui, pk.y)));
+    if (last)
+    {
+        v.x = rfma(a.ushift, rfma(-ui, pk.y, pk.x), v.x);
+        v.y = rfma(a.ushift, rfma(ui, pk.x, pk.y), v.y);
+    }
+    return v;
+}
+
+template <int K> __global__ void __launch_bounds__(tile::HT, tile_min_blocks<double>()) exact_tile(const ExactArgs a, int m)
+{
+    pdl_begin(); // before any global-memory access (programmatic launch)
+    constexpr int R = tile::R;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cx<double>* sm = reinterpret_cast<cx<double>*>(smraw);
+    cx<double>* tw = sm + tile::SLOT;
+    const int t = threadIdx.x;
+    const long long M = 1LL << m;
+    const long long base = ((long long)blockIdx.x << 11) + t; // flat over the products
+    const long long g = (long long)blockIdx.x & ((1LL << (m - 11)) - 1);
+    const long long WM = a.W * M;
+    cx<double> pk[R], x[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) pk[r] = a.spec[K * WM + base + (r << 7)];
+    tile::stage_twiddles<false>(tw, a.roots, g, t, 0);
+#pragma unroll
+    for (int r = 0; r < R; r++) x[r] = a.spec[base + (r << 7)];
+    __syncthreads();
+    tile::forward<double>(pk, sm, tw, t);
+    __syncthreads(); // the parked operand's last transpose is read
+    // U of the thread's points j = 2048 g + 16 t + r: coalesced in the permuted order
+    const cx<double>* up = a.uspec + (m > EBITS ? ((g >> 1) << EBITS) + ((g & 1) << 7) + t : (g << 11) + 16 * t);
+    const int us = m > EBITS ? 256 : 1;
+#pragma unroll
+    for (int l = 0; l < K; l++)
+    {
+        if (l > 0)
         {
 #pragma unroll
-            for (int h = 0; h < nt; h += 2)
-            {
-                const float4 v = __ldg(reinterpret_cast<const float4*>(p0 + h));
-                wk[h] = mk<float>(v.x, v.y);
-                wk[h + 1] = mk<float>(v.z, v.w);
-            }
+            for (int r = 0; r < R; r++) x[r] = a.spec[l * WM + base + (r << 7)];
+        }
+        tile::forward<double>(x, sm, tw, t); // first writes the positions this thread read last
+        if (a.cen == 0)
+        {
+#pragma unroll
+            for (int r = 0; r < R; r++) x[r] = cmul<double>(x[r], pk[r]);
         }
         else
         {
 #pragma unroll
-            for (int h = 0; h < nt; h++) wk[h] = ldg<float>(p0 + h);
+            for (int r = 0; r < R; r++) x[r] = exact_product(x[r], pk[r], a, __ldg(&up[r * us].y), l == K - 1);
         }
-    }
+        tile::inverse<double>(x, sm, tw, t);
 #pragma unroll
-    for (int k = 0; k < RB; k++)
+        for (int r = 0; r < R; r++) a.spec[l * WM + base + (r << 7)] = x[r];
+    }
+}
+
+// ---------------------------------------------------------------------------
+// whole products of 2^m-point transforms, m = 4 .. 12: 2^(11-m) to a CTA of 128
+// threads, one of 4096 points to a CTA of 256
+// ---------------------------------------------------------------------------
+// Two CTAs per SM (one at 4096 points) where a thread holds 16 twist factors of its
+// own; three below, where they repeat.
+template <int m, int K>
+__global__ void __launch_bounds__(m == 12 ? 256 : 128, m == 12 ? 1 : m == 11 ? 2 : 3) exact_single(const ExactArgs a)
+{
+    pdl_begin(); // before any global-memory access (programmatic launch)
+    using tl = TileOf<m == 12 ? 12 : 11>;
+    constexpr int R = tl::R, HT = tl::HT;
+    constexpr int M = 1 << m;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cx<double>* sm = reinterpret_cast<cx<double>*>(smraw);
+    cx<double>* tw = sm + tl::SLOT;
+    const int t = threadIdx.x;
+    const long long p0 = (long long)blockIdx.x << (m == 12 ? 0 : 11 - m); // first product of this CTA
+    const long long left = (a.W - p0) << m;                 // points of the batch from there on
+    // register r: point e = t + r HT, product p0 + (e >> m), position e mod M; a
+    // row has 2M coefficients, so the coefficient is at 2e - (e mod M), and + M
+    auto at = [&](int r) {
+        const int e = t + r * HT;
+        return 2 * e - (e & (M - 1));
+    };
+    auto load = [&](cx<double> (&x)[16], const int32_t* src, auto digit) {
+        const cx<double>* tws = fresh(a.twist);
+        constexpr int Q = m >= 10 ? 4 : 8; // points at a time: as many loads in flight as registers allow
+#pragma unroll
+        for (int h = 0; h < R; h += Q)
+        {
+            int v0[Q], v1[Q];
+#pragma unroll
+            for (int q = 0; q < Q; q++)
+            {
+                const bool ok = t + (h + q) * HT < left;
+                v0[q] = ok ? __ldg(src + p0 * 2 * M + at(h + q)) : 0;
+                v1[q] = ok ? __ldg(src + p0 * 2 * M + at(h + q) + M) : 0;
+            }
+#pragma unroll
+            for (int q = 0; q < Q; q++)
+                x[h + q] = cmul<double>(mk<double>(int_f64(digit(v0[q])), int_f64(digit(v1[q]))),
+                                        ldg<double>(tws + ((t + (h + q) * HT) & (M - 1))));
+        }
+    };
+    cx<double> pk[R];
+    load(pk, a.b, [&](int v) { return (int)((long long)v - a.cen); });
+    tl::template stage_twiddles<(m < 11)>(tw, a.roots, 0, t, M / 2);
+    __syncthreads();
+    tl::template forward<double, m>(pk, sm, tw, t);
+    __syncthreads(); // the parked operand's last transpose is read
+    ExactErr err;
+    long long* dst = reinterpret_cast<long long*>(a.c) + p0 * 2 * M;
+#pragma unroll
+    for (int l = 0; l < K; l++)
     {
-        const int pb = FWD ? (A + RB - 1 - k) : (A + k);
-        const int nt = 1 << (3 - pb);
+        cx<double> x[R];
+        load(x, a.a, [&](int v) { return exact_digit<K>(v, a.voff, l, a.w); });
+        tl::template forward<double, m>(x, sm, tw, t); // first writes the positions this thread read last
+        if (a.cen == 0)
+        {
+#pragma unroll
+            for (int r = 0; r < R; r++) x[r] = cmul<double>(x[r], pk[r]);
+        }
+        else
+        {
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                x[r] = exact_product(x[r], pk[r], a, __ldg(&a.uspec[(16 * t + r) & (M - 1)].y), l == K - 1);
+        }
+        tl::template inverse<double, m>(x, sm, tw, t);
+        const int sh = a.w * l;
+        const cx<double>* tws = fresh(a.twist);
 #pragma unroll
         for (int r = 0; r < R; r++)
         {
-            if (r & (1 << pb)) continue;
-            const cx<float> wt = w[nt - 1 + (r >> (pb + 1))];
-            if (FWD)
-                ct_bfly<float>(x[r], x[r | (1 << pb)], wt);
+            const int j = (t + r * HT) & (M - 1);
+            const cx<double> u = ldg<double>(tws + j);
+            const cx<double> v = cmul<double>(x[r], mk<double>(u.x * a.scale, -u.y * a.scale));
+            const double r0 = __dadd_rn(v.x, RND64), r1 = __dadd_rn(v.y, RND64);
+            if (t + r * HT >= left) continue;
+            err.add(__dsub_rn(v.x, __dsub_rn(r0, RND64)), v.x);
+            err.add(__dsub_rn(v.y, __dsub_rn(r1, RND64)), v.y);
+            unsigned long long i0 = (unsigned long long)(__double_as_longlong(r0) - RND64_BITS) << sh;
+            unsigned long long i1 = (unsigned long long)(__double_as_longlong(r1) - RND64_BITS) << sh;
+            if (l == 0)
+            {
+                i0 += (unsigned long long)exact_uu(a.cen, j, 2 * M);
+                i1 += (unsigned long long)exact_uu(a.cen, j + M, 2 * M);
+            }
             else
-                gs_bfly<float>(x[r], x[r | (1 << pb)], wt);
-        }
-    }
-}
-
-template <int W> __device__ __forceinline__ void slot_load(cx<float> (&x)[R], const cx<float>* sl, const SlotAddr<W>& ad)
-{
-#pragma unroll
-    for (int r = 0; r < R; r++) x[r] = sl[ad(r)];
-}
-template <int W> __device__ __forceinline__ void slot_store(const cx<float> (&x)[R], cx<float>* sl, const SlotAddr<W>& ad)
-{
-#pragma unroll
-    for (int r = 0; r < R; r++) sl[ad(r)] = x[r];
-}
-
-constexpr int NTEAM = 6;        // teams of HT threads (768 threads, 80 registers each)
-constexpr int NTT = NTEAM * HT; // threads per CTA
-
-// slots, the staged twiddles (window 0, then windows 7 and 3) of the forward
-// and of the inverse tile, one mbarrier per slot, the queue counter and the
-// teams' items
-constexpr size_t smem_bytes(int k)
-{
-    return (size_t)(2 * k) * SLOT * sizeof(float2) + 2 * (size_t)W0_PAIRS * sizeof(float4) +
-           2 * (size_t)W37_ENTRIES * sizeof(float2) + (size_t)(2 * k) * 8 + 64;
-}
-
-} // namespace stile
-
-// Timeouts of the tile kernel's bounded waits (read and cleared by
-// gpufft_split_wait_timeouts in gf_split_tile.cu, the one file that includes
-// this header).
-static __device__ unsigned g_split_wait_timeouts;
-
-template <int K>
-__global__ void __launch_bounds__(stile::NTT, 1) split_tile_kernel(const SplitArgs a, long long tiles)
-{
-    pdl_begin(); // before any global-memory access (programmatic launch)
-    using namespace stile;
-    constexpr int NS = 2 * K;     // slots: limbs of A then B
-    constexpr int NG = 2 * K - 1; // limb groups
-    extern __shared__ __align__(16) unsigned char smraw[];
-    cx<float>* slot = reinterpret_cast<cx<float>*>(smraw);
-    float4* twf = reinterpret_cast<float4*>(slot + NS * SLOT); // window-0 twiddles of the forward tile
-    float4* twi = twf + W0_PAIRS;                             // ... and of the inverse tile
-    cx<float>* tof = reinterpret_cast<cx<float>*>(twi + W0_PAIRS); // windows 7 and 3, forward tile
-    cx<float>* toi = tof + W37_ENTRIES;                             // ... inverse tile
-    unsigned long long* bar = reinterpret_cast<unsigned long long*>(toi + W37_ENTRIES);
-    int* ctl = reinterpret_cast<int*>(bar + NS); // [0] queue counter, [4 + team] the team's current item
-
-    const int tid = threadIdx.x;
-    const int team = tid >> 7;
-    const int t = tid & (HT - 1);
-    const int tbar = 1 + team; // the team's named barrier
-    const long long M = 1LL << a.geo.m;
-    const int lg_tiles = a.geo.m - LT; // log2 tiles per transform
-    const long long G = gridDim.x;
-    const bool vec = (reinterpret_cast<uintptr_t>(a.roots) & 15) == 0 &&
-                     (reinterpret_cast<uintptr_t>(a.inv_roots) & 15) == 0;
-    const SlotAddr<7> a7(t);
-    const SlotAddr<3> a3(t);
-    const SlotAddr<0> a0(t);
-
-    if (tid == 0)
-    {
-#pragma unroll
-        for (int i = 0; i < NS; i++) mbar_init(&bar[i], 1);
-        fence_mbar_init();
-        ctl[0] = 0;
-    }
-    if (blockIdx.x < tiles)
-    {
-        const long long T0 = (long long)blockIdx.x & ((1LL << lg_tiles) - 1);
-        stage_w0(twf, a.roots, T0, tid, NTT, vec);
-        stage_w37(tof, a.roots, T0, tid, NTT);
-    }
-    __syncthreads();
-
-    auto issue = [&](long long tile, int tau) {
-        const long long p = tile >> lg_tiles, T = tile & ((1LL << lg_tiles) - 1);
-        const cx<float>* src = a.spec + ((long long)tau * a.W + p) * M + (T << LT);
-        mbar_arrive_expect_tx(&bar[tau], P * sizeof(float2));
-        bulk_g2s(slot + (long long)tau * SLOT, src, P * sizeof(float2), &bar[tau]);
-    };
-
-    // The last forward stage of limb tau of `tile`: wait for its copy (bounded),
-    // then the eleven stages in place. Returns false (uniformly over the team)
-    // when the wait ran out.
-    auto forward_item = [&](long long tile, int tau, unsigned parity) -> bool {
-        const bool ok = mbar_wait_bounded(&bar[tau], parity);
-        if (bar_any(tbar, HT, !ok)) return false;
-        const long long T = tile & ((1LL << lg_tiles) - 1);
-        cx<float>* sl = slot + tau * SLOT;
-        cx<float> x[R];
-#pragma unroll
-        for (int r = 0; r < R; r++) x[r] = sl[t + (r << 7)]; // unpadded natural order, as copied
-        round<true, 7, 7, 11>(x, a.roots, T, ebase<7>(t), vec, nullptr, t, tof);
-        bar_named(tbar, HT); // the team has read the natural order
-        slot_store<7>(x, sl, a7);
-        bar_named(tbar, HT);
-        slot_load<3>(x, sl, a3);
-        round<true, 3, 3, 7>(x, a.roots, T, ebase<3>(t), vec, nullptr, t, tof);
-        slot_store<3>(x, sl, a3); // the positions this thread read
-        bar_named(tbar, HT);
-        slot_load<0>(x, sl, a0);
-        round<true, 0, 0, 3>(x, a.roots, T, ebase<0>(t), vec, twf, t);
-        slot_store<0>(x, sl, a0);
-        return true;
-    };
-
-    // The first inverse stages of group s of `tile`, in place, then the group
-    // tile to the workspace; the slot's copy for `next` starts once the team
-    // has read it.
-    auto inverse_item = [&](long long tile, int s, long long next) {
-        const long long p = tile >> lg_tiles, T = tile & ((1LL << lg_tiles) - 1);
-        cx<float>* sl = slot + s * SLOT;
-        cx<float> x[R];
-        slot_load<0>(x, sl, a0);
-        round<false, 0, 0, 3>(x, a.inv_roots, T, ebase<0>(t), vec, twi, t);
-        slot_store<0>(x, sl, a0);
-        bar_named(tbar, HT);
-        slot_load<3>(x, sl, a3);
-        round<false, 3, 3, 7>(x, a.inv_roots, T, ebase<3>(t), vec, nullptr, t, toi);
-        slot_store<3>(x, sl, a3);
-        bar_named(tbar, HT);
-        slot_load<7>(x, sl, a7);
-        bar_named(tbar, HT); // the team has read slot s
-        if (next >= 0 && t == 0)
-        {
-            fence_proxy_async();
-            issue(next, s);
-        }
-        round<false, 7, 7, 11>(x, a.inv_roots, T, ebase<7>(t), vec, nullptr, t, toi);
-        cx<float>* dst = a.group + ((long long)s * a.W + p) * M + (T << LT) + t;
-#pragma unroll
-        for (int r = 0; r < R; r++) dst[r << 7] = x[r];
-    };
-
-    // Draw items from the queue until it is empty: items [0, n_inv) are the
-    // inverse items of `tile`, the next n_fwd the forward items of `ftile`.
-    // Returns false if a forward wait of this team ran out.
-    auto run_queue = [&](long long tile, int n_inv, long long ftile, int n_fwd, unsigned fpar,
-                         long long next) -> bool {
-        bool ok = true;
-        for (;;)
-        {
-            if (t == 0) ctl[4 + team] = atomicAdd(&ctl[0], 1);
-            bar_named(tbar, HT);
-            const int item = ctl[4 + team];
-            bar_named(tbar, HT); // every thread has the item before the leader draws again
-            if (item >= n_inv + n_fwd) break;
-            if (item < n_inv)
-                inverse_item(tile, item, next);
-            else if (ok)
-                ok = forward_item(ftile, item - n_inv, fpar);
-        }
-        return ok;
-    };
-
-    long long tile = blockIdx.x;
-    if (tid == 0)
-        for (int tau = 0; tau < NS; tau++) issue(tile, tau);
-    bool ok = run_queue(-1, 0, tile, NS, 0u, -1);
-    for (unsigned it = 0;; it++)
-    {
-        // every limb spectrum of `tile` is in its slot (or some team's wait ran out)
-        if (__syncthreads_or(ok ? 0 : 1))
-        {
-            if (tid == 0)
             {
-                // all copies of this iteration were issued: drain them (bounded)
-                for (int tau = 0; tau < NS; tau++) (void)mbar_wait_bounded(&bar[tau], it & 1);
-                atomicAdd(&g_split_wait_timeouts, 1u);
-                if (a.max_err) atomicMax(a.max_err, 0x7f800000u); // +inf: the call's result is not certified
+                // the sum so far is this thread's own store
+                i0 += (unsigned long long)dst[at(r)];
+                i1 += (unsigned long long)dst[at(r) + M];
             }
-            return;
+            dst[at(r)] = (long long)i0;
+            dst[at(r) + M] = (long long)i1;
         }
-        const long long T = tile & ((1LL << lg_tiles) - 1);
-        // ---- group sums at every point, over slots 0 .. NG-1 ----
-        {
-            const float uscale = (float)(1 << a.ur);
-#pragma unroll 1
-            for (int e = tid; e < P; e += NTT)
-            {
-                const int ad = ppos(e);
-                cx<float> v[NS];
-#pragma unroll
-                for (int tau = 0; tau < NS; tau++) v[tau] = slot[tau * SLOT + ad];
-                // A_i B_j accumulated with paired fused multiply-adds:
-                // (a.x, a.x) (b.x, b.y) + (a.y, a.y) (-b.y, b.x), the pairs formed
-                // once per limb
-                float2 ax[K], ay[K], bs[K];
-#pragma unroll
-                for (int l = 0; l < K; l++)
-                {
-                    ax[l] = make_float2(v[l].x, v[l].x);
-                    ay[l] = make_float2(v[l].y, v[l].y);
-                    bs[l] = make_float2(-v[K + l].y, v[K + l].x);
-                }
-                cx<float> acc[NG];
-#pragma unroll
-                for (int sg = 0; sg < NG; sg++)
-                {
-                    acc[sg] = mk<float>(0.f, 0.f);
-#pragma unroll
-                    for (int i2 = 0; i2 < K; i2++)
-                        if (sg - i2 >= 0 && sg - i2 < K)
-                        {
-                            acc[sg] = __ffma2_rn(ax[i2], v[K + sg - i2], acc[sg]);
-                            acc[sg] = __ffma2_rn(ay[i2], bs[sg - i2], acc[sg]);
-                        }
-                }
-                if (a.K)
-                {
-                    // U is stored in the 4096-point-tile permuted order of the table block
-                    const long long j = (T << LT) + e;
-                    const long long ju = (M > 4096) ? ((j & ~4095LL) | ((j & 4095) >> 4) | ((j & 15) << 8)) : j;
-                    const cx<float> u = ldg<float>(a.uspec + ju);
-                    cx<float> cen[K];
-#pragma unroll
-                    for (int l = 0; l < K; l++)
-                    {
-                        cx<float> ee = cadd<float>(v[l], v[K + l]);
-                        if (l < K - 1) ee = cadd<float>(ee, u);
-                        cen[l] = cmul<float>(mk<float>(ee.x * uscale, ee.y * uscale), u);
-                    }
-                    // limb l's term joins group l + uq: one uniform branch, compile-time indices
-                    auto add_from = [&](auto q) {
-                        constexpr int Q = decltype(q)::value;
-#pragma unroll
-                        for (int l = 0; l < K; l++)
-                            if (l + Q < NG) acc[l + Q] = cadd<float>(acc[l + Q], cen[l]);
-                    };
-                    static_assert(K <= 6, "the switch below covers uq <= 6");
-                    switch (a.uq)
-                    {
-                    case 0: add_from(std::integral_constant<int, 0>{}); break;
-                    case 1: add_from(std::integral_constant<int, 1>{}); break;
-                    case 2: add_from(std::integral_constant<int, 2>{}); break;
-                    case 3: add_from(std::integral_constant<int, 3>{}); break;
-                    case 4: add_from(std::integral_constant<int, 4>{}); break;
-                    case 5: add_from(std::integral_constant<int, 5>{}); break;
-                    case 6: add_from(std::integral_constant<int, 6>{}); break;
-                    default: break;
-                    }
-                }
-#pragma unroll
-                for (int sg = 0; sg < NG; sg++) slot[sg * SLOT + ad] = acc[sg];
-            }
-        }
-        const long long next = tile + G;
-        const bool has_next = next < tiles;
-        // window-0 twiddles: the inverse items of this tile and the forward items
-        // of the next (the previous tile's inverse and this tile's forward items
-        // are done)
-        stage_w0(twi, a.inv_roots, T, tid, NTT, vec);
-        stage_w37(toi, a.inv_roots, T, tid, NTT);
-        if (has_next)
-        {
-            stage_w0(twf, a.roots, next & ((1LL << lg_tiles) - 1), tid, NTT, vec);
-            stage_w37(tof, a.roots, next & ((1LL << lg_tiles) - 1), tid, NTT);
-        }
-        if (tid == 0) ctl[0] = 0; // the queue restarts
-        __syncthreads();
-        // slot NS-1 held a limb only: the next tile's copy can start now
-        if (has_next && tid == 0)
-        {
-            fence_proxy_async();
-            issue(next, NS - 1);
-        }
-        ok = run_queue(tile, NG, next, has_next ? NS : 0, (it + 1) & 1, has_next ? next : -1);
-        if (!has_next) break;
-        tile = next;
     }
+    report_err(a.max_err, err.value());
 }
 
 } // namespace gfb

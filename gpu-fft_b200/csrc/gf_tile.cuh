@@ -39,138 +39,196 @@
 
 namespace gfb
 {
-namespace tile
-{
-constexpr int LT = 11;            // log2 points per tile
-constexpr int P = 1 << LT;        // 2048 points
-constexpr int HT = 128;           // threads
-constexpr int R = P / HT;         // 16 points per thread
-constexpr int SLOT = P + P / 16;  // padded transpose buffer
-constexpr int S0 = HT + 1;        // stride of the staged innermost twiddles
-constexpr int S3 = 9;             // stride of the staged middle twiddles
-constexpr int TWN = 7 * S0 + 16 * S3 + 8;
 
-// e of register 0 of thread t when the registers are the e-bits [W, W+4)
-template <int W> __device__ __forceinline__ int ebase(int t)
+// One tile of 2^LT points on 2^LT / 16 threads: LT = 11 as above; LT = 12 (256
+// threads, rounds on the e-bits [8,12), [4,8), [0,4)) for whole transforms of 4096
+// points (gf_single.cuh).
+template <int LT> struct TileOf
 {
-    return (t & ((1 << W) - 1)) | ((t >> W) << (W + 4));
-}
-__device__ __forceinline__ constexpr int ppos(int e) { return e + (e >> 4); }
-// ppos(ebase + (r << W)) - ppos(ebase): the window bits of ebase are clear
-template <int W> __device__ __forceinline__ constexpr int poff(int r) { return (r << W) + ((r << W) >> 4); }
+    static constexpr int P = 1 << LT;           // points
+    static constexpr int R = 16;                // points per thread
+    static constexpr int HT = P / R;            // threads
+    static constexpr int SLOT = P + P / 16;     // padded transpose buffer
+    static constexpr int W1 = LT - 4, W2 = LT - 8, HI0 = LT - 8; // windows of the rounds, bits of the last
+    static_assert(LT == 11 || LT == 12, "three rounds");
+    static constexpr int N0 = HI0 == 4 ? 8 : 7; // even twiddles per thread of the innermost round
+    static constexpr int S0 = HT + 1;           // stride of the staged innermost twiddles
+    static constexpr int S2 = 9;                // stride of the staged middle twiddles
+    static constexpr int TWN = N0 * S0 + 16 * S2 + 8;
 
-template <int W, typename C> __device__ __forceinline__ void put(const C (&x)[R], C* sm, int t)
-{
-    const int b = ppos(ebase<W>(t));
-#pragma unroll
-    for (int r = 0; r < R; r++) sm[b + poff<W>(r)] = x[r];
-}
-template <int W, typename C> __device__ __forceinline__ void get(C (&x)[R], const C* sm, int t)
-{
-    const int b = ppos(ebase<W>(t));
-#pragma unroll
-    for (int r = 0; r < R; r++) x[r] = sm[b + poff<W>(r)];
-}
-
-// The tile's even twiddles. A stage with nt = 2^k >= 2 twiddles per thread uses
-// table[(T << u) + nt i + h], h < nt, for an i of the thread; the even h of the
-// stages of a round sit at positions nt/2 + h/2 (0 for the stage with one
-// twiddle, whose entry may be odd):
-//   window 7 (u = 0..3)  i = 0:       tw7[pos],             pos 0..7
-//   window 3 (u = 4..7)  i = t >> 3:  tw3[(t >> 3) S3 + pos], pos 0..7
-//   window 0 (u = 8..10) i = t:       tw0[(pos - 1) S0 + t],  pos 1..7
-template <typename C> __device__ __forceinline__ void stage_twiddles(C* tw, const C* __restrict__ tab, long long T, int t)
-{
-    C* tw0 = tw;
-    C* tw3 = tw + 7 * S0;
-    C* tw7 = tw3 + 16 * S3;
-    // window 0: linear even entry p of stage u is table[(T << u) + 2p]
-#pragma unroll
-    for (int k = 0; k < 7; k++)
+    // e of register 0 of thread t when the registers are the e-bits [W, W+4)
+    template <int W> static __device__ __forceinline__ int ebase(int t)
     {
-        const int p = (k == 0 ? 0 : k < 3 ? (k - 1) * HT : (k - 3) * HT) + t; // of stage 8, 9 or 10
-        const int lg = k == 0 ? 0 : k < 3 ? 1 : 2;                           // log2 evens per thread
-        const int i = p >> lg, pos = (1 << lg) + (p & ((1 << lg) - 1));
-        tw0[(pos - 1) * S0 + i] = __ldg(tab + (T << (8 + lg)) + 2 * p);
+        return (t & ((1 << W) - 1)) | ((t >> W) << (W + 4));
     }
-    // window 3: 16 i x 8 positions
-    {
-        const int i = t >> 3, pos = t & 7;
-        const int lg = pos == 0 ? 0 : 32 - __clz(pos); // log2 twiddles per thread of the stage
-        const int h = pos == 0 ? 0 : 2 * (pos - (1 << (lg - 1)));
-        tw3[i * S3 + pos] = __ldg(tab + (T << (4 + lg)) + (i << lg) + h);
-    }
-    if (t < 8)
-    {
-        const int lg = t == 0 ? 0 : 32 - __clz(t);
-        const int h = t == 0 ? 0 : 2 * (t - (1 << (lg - 1)));
-        tw7[t] = __ldg(tab + (T << lg) + h);
-    }
-}
+    static __device__ __forceinline__ constexpr int ppos(int e) { return e + (e >> 4); }
+    // ppos(ebase + (r << W)) - ppos(ebase): the window bits of ebase are clear
+    template <int W> static __device__ __forceinline__ constexpr int poff(int r) { return (r << W) + ((r << W) >> 4); }
 
-// One round on the register bits [LO, HI): the stage on bit pb has 2^(3-pb)
-// twiddles per thread. `tw` points to the thread's entry of position 0, `st` is
-// the distance between positions.
-template <typename T, bool FWD, int LO, int HI>
-__device__ __forceinline__ void round(cx<T> (&x)[R], const cx<T>* tw, int st)
-{
-#pragma unroll
-    for (int k = 0; k < HI - LO; k++)
+    template <int W, typename C> static __device__ __forceinline__ void put(const C (&x)[R], C* sm, int t)
     {
-        const int pb = FWD ? HI - 1 - k : LO + k;
-        const int nt = 1 << (3 - pb); // twiddles of this stage per thread
-        cx<T> e[4];
+        const int b = ppos(ebase<W>(t));
 #pragma unroll
-        for (int i = 0; i < (nt > 1 ? nt / 2 : 1); i++)
+        for (int r = 0; r < R; r++) sm[b + poff<W>(r)] = x[r];
+    }
+    template <int W, typename C> static __device__ __forceinline__ void get(C (&x)[R], const C* sm, int t)
+    {
+        const int b = ppos(ebase<W>(t));
+#pragma unroll
+        for (int r = 0; r < R; r++) x[r] = sm[b + poff<W>(r)];
+    }
+
+    // The tile's even twiddles. A stage with nt = 2^k twiddles per thread uses
+    // table[(T << u) + nt i + h], h < nt, for an i of the thread; the even h of the
+    // stages of a round sit at positions nt/2 + h/2 (0 for the stage with one
+    // twiddle, whose entry may be odd):
+    //   outer round   (u = 0..3)  i = 0:
+    //   middle round  (u = 4..7)  i = t >> W2
+    //   inner round   (u = 8..)   i = t (LT = 11 has no stage with one twiddle here)
+    template <typename C> static __device__ __forceinline__ C* outer(C* tw) { return tw + N0 * S0 + 16 * S2; }
+    template <typename C> static __device__ __forceinline__ C* middle(C* tw, int i) { return tw + N0 * S0 + i * S2; }
+    template <typename C> static __device__ __forceinline__ C* inner(C* tw, int i) { return tw + (N0 - 8) * S0 + i; }
+
+    // SHORT: whole transforms shorter than the tile have a shorter table (`entries`)
+    // and use no others
+    template <bool SHORT, typename C>
+    static __device__ __forceinline__ void stage_twiddles(C* tw, const C* __restrict__ tab, long long T, int t, long long entries)
+    {
+        // inner round: linear even entry p of a stage is table[(T << u) + 2p]
+        if constexpr (HI0 == 4) inner(tw, t)[0] = __ldg(tab + (T << 8) + t);
+#pragma unroll
+        for (int k = 0; k < 7; k++)
         {
-            e[i] = tw[((nt >> 1) + i) * st];
-            if (!FWD) e[i].y = -e[i].y; // inverse root
+            const int p = (k == 0 ? 0 : k < 3 ? (k - 1) * HT : (k - 3) * HT) + t; // of one of the last three stages
+            const int lg = k == 0 ? 0 : k < 3 ? 1 : 2;                           // log2 evens per thread
+            const long long e = (T << (LT - 3 + lg)) + 2 * p;
+            if (!SHORT || e < entries) inner(tw, p >> lg)[((1 << lg) + (p & ((1 << lg) - 1))) * S0] = __ldg(tab + e);
         }
-#pragma unroll
-        for (int r = 0; r < R; r++)
+        // middle round: 16 i x 8 positions
+        if (HT == 128 || t < 128)
         {
-            if (r & (1 << pb)) continue;
-            const int h = r >> (pb + 1);
-            const cx<T> ev = e[h >> 1];
-            const cx<T> w = !(h & 1) ? ev : (FWD ? mk<T>(-ev.y, ev.x) : mk<T>(ev.y, -ev.x));
-            if (FWD)
-                ct_bfly<T>(x[r], x[r | (1 << pb)], w);
-            else
-                gs_bfly<T>(x[r], x[r | (1 << pb)], w);
+            const int i = t >> 3, pos = t & 7;
+            const int lg = pos == 0 ? 0 : 32 - __clz(pos); // log2 twiddles per thread of the stage
+            const int h = pos == 0 ? 0 : 2 * (pos - (1 << (lg - 1)));
+            const long long e = (T << (4 + lg)) + (i << lg) + h;
+            if (!SHORT || e < entries) middle(tw, i)[pos] = __ldg(tab + e);
+        }
+        if (t < 8)
+        {
+            const int lg = t == 0 ? 0 : 32 - __clz(t);
+            const int h = t == 0 ? 0 : 2 * (t - (1 << (lg - 1)));
+            const long long e = (T << lg) + h;
+            if (!SHORT || e < entries) outer(tw)[t] = __ldg(tab + e);
         }
     }
-}
 
-// Eleven forward stages: x in window 7, out in window 0. The caller has made
-// sure that no thread still reads the buffer.
-template <typename T> __device__ __forceinline__ void forward(cx<T> (&x)[R], cx<T>* sm, const cx<T>* tw, int t)
-{
-    round<T, true, 0, 4>(x, tw + 7 * S0 + 16 * S3, 1);
-    put<7>(x, sm, t);
-    __syncthreads();
-    get<3>(x, sm, t);
-    round<T, true, 0, 4>(x, tw + 7 * S0 + (t >> 3) * S3, 1);
-    put<3>(x, sm, t); // the positions this thread read
-    __syncthreads();
-    get<0>(x, sm, t);
-    round<T, true, 0, 3>(x, tw - S0 + t, S0);
-}
+    // One round on the register bits [LO, HI): the stage on bit pb has 2^(3-pb)
+    // twiddles per thread. `tw` points to the thread's entry of position 0, `st` is
+    // the distance between positions.
+    template <typename T, bool FWD, int LO, int HI>
+    static __device__ __forceinline__ void round(cx<T> (&x)[R], const cx<T>* tw, int st)
+    {
+#pragma unroll
+        for (int k = 0; k < HI - LO; k++)
+        {
+            const int pb = FWD ? HI - 1 - k : LO + k;
+            const int nt = 1 << (3 - pb); // twiddles of this stage per thread
+            cx<T> e[4];
+#pragma unroll
+            for (int i = 0; i < (nt > 1 ? nt / 2 : 1); i++)
+            {
+                e[i] = tw[((nt >> 1) + i) * st];
+                if (!FWD) e[i].y = -e[i].y; // inverse root
+            }
+#pragma unroll
+            for (int r = 0; r < R; r++)
+            {
+                if (r & (1 << pb)) continue;
+                const int h = r >> (pb + 1);
+                const cx<T> ev = e[h >> 1];
+                const cx<T> w = !(h & 1) ? ev : (FWD ? mk<T>(-ev.y, ev.x) : mk<T>(ev.y, -ev.x));
+                if (FWD)
+                    ct_bfly<T>(x[r], x[r | (1 << pb)], w);
+                else
+                    gs_bfly<T>(x[r], x[r | (1 << pb)], w);
+            }
+        }
+    }
 
-// Eleven inverse stages: x in window 0 (its positions of the buffer are this
-// thread's), out in window 7.
-template <typename T> __device__ __forceinline__ void inverse(cx<T> (&x)[R], cx<T>* sm, const cx<T>* tw, int t)
-{
-    round<T, false, 0, 3>(x, tw - S0 + t, S0);
-    put<0>(x, sm, t);
-    __syncthreads();
-    get<3>(x, sm, t);
-    round<T, false, 0, 4>(x, tw + 7 * S0 + (t >> 3) * S3, 1);
-    put<3>(x, sm, t);
-    __syncthreads();
-    get<7>(x, sm, t);
-    round<T, false, 0, 4>(x, tw + 7 * S0 + 16 * S3, 1);
-}
-} // namespace tile
+    // The round of window W on its HI lowest bits, for 2^m-point transforms side by
+    // side in the tile (m = LT: one transform, or one tile of a longer one): only
+    // the stages on e-bits below m, with the group index taken inside the transform.
+    // With m < W + 4 the registers' upper bits number sub-networks and the twiddles
+    // are table[0 .. 8).
+    template <typename T, bool FWD, int W, int HI, int m>
+    static __device__ __forceinline__ void round_m(cx<T> (&x)[R], cx<T>* tw, int t)
+    {
+        if constexpr (m >= W + 4)
+        {
+            constexpr int mask = (1 << (m - 4 - W)) - 1;
+            if constexpr (W == W1) round<T, FWD, 0, HI>(x, outer(tw), 1);
+            else if constexpr (W == W2) round<T, FWD, 0, HI>(x, middle(tw, (t >> W2) & mask), 1);
+            else round<T, FWD, 0, HI>(x, inner(tw, t & mask), S0);
+        }
+        else if constexpr (m > W)
+        {
+            constexpr int NB = m - W;
+#pragma unroll
+            for (int k = 0; k < NB; k++)
+            {
+                const int pb = FWD ? NB - 1 - k : k;
+                const int nt = 1 << (NB - 1 - pb); // twiddles of the stage: table[0 .. nt)
+#pragma unroll
+                for (int r = 0; r < R; r++)
+                {
+                    if (r & (1 << pb)) continue;
+                    const int h = (r >> (pb + 1)) & (nt - 1);
+                    cx<T> ev = outer(tw)[4 + (h >> 1)];
+                    if (!FWD) ev.y = -ev.y;
+                    const cx<T> w = !(h & 1) ? ev : (FWD ? mk<T>(-ev.y, ev.x) : mk<T>(ev.y, -ev.x));
+                    if (FWD)
+                        ct_bfly<T>(x[r], x[r | (1 << pb)], w);
+                    else
+                        gs_bfly<T>(x[r], x[r | (1 << pb)], w);
+                }
+            }
+        }
+    }
+
+    // Forward stages: x in window W1, out in window 0. The caller has made sure that
+    // no thread still reads the buffer.
+    template <typename T, int m = LT>
+    static __device__ __forceinline__ void forward(cx<T> (&x)[R], cx<T>* sm, cx<T>* tw, int t)
+    {
+        round_m<T, true, W1, 4, m>(x, tw, t);
+        put<W1>(x, sm, t);
+        __syncthreads();
+        get<W2>(x, sm, t);
+        round_m<T, true, W2, 4, m>(x, tw, t);
+        put<W2>(x, sm, t); // the positions this thread read
+        __syncthreads();
+        get<0>(x, sm, t);
+        round_m<T, true, 0, HI0, m>(x, tw, t);
+    }
+
+    // Inverse stages: x in window 0 (its positions of the buffer are this thread's),
+    // out in window W1.
+    template <typename T, int m = LT>
+    static __device__ __forceinline__ void inverse(cx<T> (&x)[R], cx<T>* sm, cx<T>* tw, int t)
+    {
+        round_m<T, false, 0, HI0, m>(x, tw, t);
+        put<0>(x, sm, t);
+        __syncthreads();
+        get<W2>(x, sm, t);
+        round_m<T, false, W2, 4, m>(x, tw, t);
+        put<W2>(x, sm, t);
+        __syncthreads();
+        get<W1>(x, sm, t);
+        round_m<T, false, W1, 4, m>(x, tw, t);
+    }
+};
+constexpr int TILE_LT = 11;
+using tile = TileOf<TILE_LT>;
 
 enum TileMode
 {
@@ -195,23 +253,22 @@ template <typename T, int MODE>
 __global__ void __launch_bounds__(tile::HT, tile_min_blocks<T>()) tile_product_kernel(const TileArgs<T> a)
 {
     pdl_begin(); // before any global-memory access (programmatic launch)
-    using namespace tile;
-    constexpr int NOPS = MODE == TILE_VJP ? 2 : 1;
+    constexpr int NOPS = MODE == TILE_VJP ? 2 : 1, R = tile::R;
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
-    cx<T>* tw = sm + SLOT;
+    cx<T>* tw = sm + tile::SLOT;
     const int t = threadIdx.x;
-    const long long base = ((long long)blockIdx.x << LT) + t; // flat over the products
-    const long long g = (long long)blockIdx.x & ((1LL << (a.m - LT)) - 1);
+    const long long base = ((long long)blockIdx.x << 11) + t; // flat over the products
+    const long long g = (long long)blockIdx.x & ((1LL << (a.m - 11)) - 1);
     // both operands' loads are in flight before the first stage
     cx<T> pk[R], x[R];
 #pragma unroll
     for (int r = 0; r < R; r++) pk[r] = a.park[base + (r << 7)];
-    stage_twiddles(tw, a.roots, g, t);
+    tile::stage_twiddles<false>(tw, a.roots, g, t, 0);
 #pragma unroll
     for (int r = 0; r < R; r++) x[r] = a.in[0][base + (r << 7)];
     __syncthreads();
-    forward<T>(pk, sm, tw, t);
+    tile::forward<T>(pk, sm, tw, t);
     __syncthreads(); // the parked operand's last transpose is read
 #pragma unroll
     for (int l = 0; l < NOPS; l++)
@@ -221,10 +278,10 @@ __global__ void __launch_bounds__(tile::HT, tile_min_blocks<T>()) tile_product_k
 #pragma unroll
             for (int r = 0; r < R; r++) x[r] = a.in[l][base + (r << 7)];
         }
-        forward<T>(x, sm, tw, t); // first writes the positions this thread read last
+        tile::forward<T>(x, sm, tw, t); // first writes the positions this thread read last
 #pragma unroll
         for (int r = 0; r < R; r++) x[r] = MODE == TILE_VJP ? cmulc<T>(pk[r], x[r]) : cmul<T>(x[r], pk[r]);
-        inverse<T>(x, sm, tw, t);
+        tile::inverse<T>(x, sm, tw, t);
 #pragma unroll
         for (int r = 0; r < R; r++) a.out[l][base + (r << 7)] = x[r];
     }

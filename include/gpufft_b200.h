@@ -341,6 +341,15 @@ size_t gpufft_negacyclic_mul_split_workspace_bytes(int n_power, int batch, int n
  * max_error (device pointer, may be NULL; the call zeroes it first) receives
  * the largest distance of any limb-group value to its nearest integer.
  *
+ * How it is computed. The plan names what the call must hold: FP32 transforms
+ * of num_limbs limbs of both operands. On B200 the same integers are cheaper on
+ * FP64 transforms with only `a` cut into one to three limbs (5 transforms
+ * instead of 19 for 24 bits), so a call whose plan is within the error model
+ * runs that way (rings N = 2^5 .. 2^17; from 2^14 on, waves of at least one
+ * 2048-point tile per SM; a 16-byte aligned workspace that also holds the
+ * FP64 twiddles, 40 N/2 bytes; results apart from the operands), and max_error
+ * reports its groups. Other calls run the FP32 limb chain.
+ *
  * What max_error certifies. Every result coefficient is exact when the
  * floating-point error of every limb-group value is below 0.5. max_error
  * measures the distance to the NEAREST integer, so it detects errors up to
@@ -349,30 +358,26 @@ size_t gpufft_negacyclic_mul_split_workspace_bytes(int n_power, int batch, int n
  * (a-priori) bound for FP32 transforms of these lengths is orders of magnitude
  * above 0.5, so exactness is statistical: the limb plan (gpufft_split_plan)
  * keeps the predicted largest error at or below 0.2, from an error model
- * calibrated on measured limb products, and the measured max_error on uniform
- * 24-bit data is about 0.13 at N = 2^16 and 0.22 at N = 2^17. Group values
- * above 2^22 report 1.0 (not certified), a timed-out internal wait reports
- * +inf (see gpufft_split_wait_timeouts). */
+ * calibrated on measured limb products (the FP64 form at or below 0.06), and
+ * the measured max_error on uniform 24-bit data is about 0.01 at N = 2^16 (0.13
+ * in the FP32 chain). Group values above 2^22 (2^50 in the FP64 form) report 1.0
+ * (not certified). */
 int gpufft_negacyclic_mul_split_f32(const int32_t* a, const int32_t* b, int64_t* c, int n_power, int batch,
                                     int input_bits, int non_negative, int limb_bits, int num_limbs,
                                     const void* tables, void* workspace, size_t workspace_bytes,
                                     float* max_error, gpufft_stream_t stream);
-/* Rings N = 2^14 .. 2^16 with at most five limbs (with a 16-byte aligned
- * workspace, and at least one 2048-point tile per SM per wave: 10 products at
- * N = 2^16) run the contiguous stages of every limb and limb group in one
- * persistent kernel that keeps a product
- * tile's limb spectra in shared memory (on = 1, the default), or in the chain
- * of separate pass and group-sum kernels (on = 0); the integers are the same.
- * A negative value only queries. Returns the previous setting. Process-wide. */
+/* The FP64 form above (on = 1, the default) or always the chain of limb passes
+ * (on = 0); the integers are the same. A negative value only queries. Returns
+ * the previous setting. Process-wide. */
 int gpufft_set_split_tile(int on);
-/* Waits of that kernel on its bulk copies are bounded (2 s); a wait that runs
- * out makes the call report max_error = +inf and is counted here. Reads the
- * count (synchronous) and clears it when `clear` is nonzero. */
+/* Bounded waits of the exact product that ran out: its kernels have none, so the
+ * count is 0. */
 int gpufft_split_wait_timeouts(unsigned* count, int clear);
 /* The same exact product with FP64 transforms, N = 2^2 .. 2^17 (no reference
  * counterpart). Its limb plan uses the FP64 error model, so it needs far fewer
  * limbs (two 12-bit limbs for 24-bit coefficients at N = 2^16). `tables` is the
- * f64 native twiddle block (gpufft_ffnt_make_tables_f64). */
+ * f64 native twiddle block (gpufft_ffnt_make_tables_f64). Runs in the form
+ * described above where it applies (one operand whole). */
 int gpufft_split_plan_f64(int n_power, int input_bits, int non_negative, int* limb_bits, int* num_limbs);
 size_t gpufft_negacyclic_mul_split_f64_workspace_bytes(int n_power, int batch, int num_limbs);
 int gpufft_negacyclic_mul_split_f64(const int32_t* a, const int32_t* b, int64_t* c, int n_power, int batch,
