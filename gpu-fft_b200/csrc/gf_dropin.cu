@@ -16,11 +16,28 @@
 namespace gfb
 {
 
+// Passes of (m - 11, 11) stages, the second on 2048-point tiles, where the column
+// pass has a kernel for the rest and two tiles per SM keep the tile pass's CTAs
+// overlapping; the plan above otherwise. FP64 FFNT calls (fold) keep 4096-point
+// tiles from three per two SMs on: one column stage fewer next to the fold, longer
+// runs under one staging of the twiddles (product, N = 2^16: batch 256 351 against
+// 413 us, batch 30 52 against 59; N = 2^15, batch 20, below the line: 36 against 34;
+// C_C N = 2^14, batch 100: 83 against 80, R_R, batch 75: 56 against 51).
+template <typename T> static Plan transform_plan(int m, long long batch, bool fold)
+{
+    Plan p = make_plan(m);
+    if (m <= EBITS || m - 11 > COL_MAX_L || (batch << (m - 11)) < 2LL * sm_count()) return p;
+    if (sizeof(T) == 8 && fold && 2 * (batch << (m - EBITS)) >= 3LL * sm_count()) return p;
+    p.L[0] = m - 11;
+    p.L[1] = 11;
+    return p;
+}
+
 template <typename T>
 static int run_forward(int m, int neg, long long batch, const void* in, int in_kind, void* out,
                        const cx<T>* table, const cx<T>* twist, int zero_pad, cudaStream_t s)
 {
-    const Plan p = make_plan(m);
+    const Plan p = transform_plan<T>(m, batch, in_kind == IN_FOLD);
     for (int k = 0; k < p.np; k++)
     {
         long long ctas = 0;
@@ -48,7 +65,7 @@ static int run_inverse(int m, int neg, long long batch, void* work, int mult, lo
                        void* out, int out_kind, const cx<T>* table, const cx<T>* untwist, cx<T> scale,
                        cudaStream_t s)
 {
-    const Plan p = make_plan(m);
+    const Plan p = transform_plan<T>(m, batch, out_kind == OUT_UNFOLD);
     for (int k = p.np - 1; k >= 0; k--)
     {
         long long ctas = 0;

@@ -782,6 +782,12 @@ static inline int launch_pass_shape(const PassArgs<T>& a, long long ctas, cudaSt
     return launch_k(pass_kernel<T, FWD, L, STRIDED, PERM>, dim3((unsigned)ctas), dim3(NTHR), smem, s, a);
 }
 
+// The tile form of a contiguous pass of LT = 11 or 12 stages (gf_tile_pass.cuh), or
+// -1 for a load or store it does not have (forward: complex rows, and for whole
+// transforms the fold and real rows; inverse: complex rows or their product, any
+// store for whole transforms).
+template <typename T> int launch_tile_pass(const PassArgs<T>& a, bool fwd, int LT, cudaStream_t s);
+
 // Launch pass k of plan p (the pass's L selects the compiled shape).
 template <typename T, bool FWD>
 static inline int launch_pass(const PassArgs<T>& a, const Plan& p, int k, long long ctas, cudaStream_t s)
@@ -836,6 +842,11 @@ static inline int launch_pass(const PassArgs<T>& a, const Plan& p, int k, long l
             c.twist = a.twist;
             c.untwist = a.twist;
             return launch_cluster_pass<T, FWD ? CLM_FWD : CLM_INV>(c, a.batch, a.batch, s, L);
+        }
+        if ((L == 11 || L == EBITS) && (a.batch << (a.geo.m - L)) >= sm_count())
+        {
+            const int st = launch_tile_pass<T>(a, FWD, L, s);
+            if (st >= 0) return st;
         }
         return dispatch_int<1, EBITS>(L, [&]<int LL>() { return launch_pass_shape<T, FWD, LL, false>(a, ctas, s); });
     }

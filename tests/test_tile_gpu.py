@@ -67,3 +67,92 @@ def test_vjp_tile_rows(gf, dev, n_power, batch):
     for got, x in ((ga, b), (gb, a)):
         want = torch.fft.irfft(G * torch.fft.rfft(x[:2].double(), 4 * n).conj(), 4 * n)[:, :n]
         assert (torch.linalg.norm(got[:2] - want) / torch.linalg.norm(want)).item() < 2e-5
+
+
+def reference_table(gf, n, dtype, dev):
+    r, ri, _ = gf.host_fft_tables(n // 2, dtype)
+    return torch.from_numpy(r).to(dev), torch.from_numpy(ri).to(dev)
+
+
+# one-pass rows of 2048 and 4096 points from one tile per SM on (148), two passes
+# (L, 11) from 296 tiles on, (L, 12) from 222 for FP64 FFNT; zero-padded and plain rows
+@pytest.mark.parametrize("n_power,batch,dtype", [
+    (12, 149, "f64"), (12, 200, "f32"), (13, 74, "f64"), (13, 75, "f32"), (13, 149, "f64"), (14, 75, "f32"),
+    (15, 28, "f64"), (16, 15, "f64"), (16, 19, "f32"), (17, 7, "f64"), (17, 10, "f32"), (18, 5, "f64")])
+def test_ffnt_tile_passes(gf, O, dev, n_power, batch, dtype):
+    n = 1 << n_power
+    T = torch.float64 if dtype == "f64" else torch.float32
+    C = torch.complex128 if dtype == "f64" else torch.complex64
+    g = torch.Generator(device=dev).manual_seed(n_power * 1000 + batch)
+    x = torch.randint(-(1 << 10), 1 << 10, (2 * batch, n), device=dev, generator=g, dtype=torch.int32).to(T)
+    roots, inv, twist, untwist = (torch.from_numpy(t).to(dev) for t in gf.host_ffnt_tables(n, dtype))
+    fwd = gf.fft_configuration(n_power=n_power, fft_type=gf.FORWARD)
+    bwd = gf.fft_configuration(n_power=n_power, fft_type=gf.INVERSE, mod_inverse=complex(2.0 / n))
+
+    def product(rows, b):
+        temp = torch.empty(2 * b * n // 2, dtype=C, device=dev)
+        out = torch.empty(b, n, dtype=T, device=dev)
+        gf.GPU_FFNT(rows, temp, twist, roots, fwd, 2 * b, False)
+        gf.GPU_FFNT(out, temp, untwist, inv, bwd, b, True)
+        return out
+
+    c = product(x, batch)
+    few = product(torch.cat([x[batch - 1: batch], x[-1:]]), 1)  # too few rows for the tiles
+    assert torch.equal(c[-1:], few)
+    idx = np.sort(np.random.default_rng(batch).choice(n, 64, replace=False)).astype(np.int32)
+    want = O.wrap64(O.negacyclic_coeffs(x[0].cpu().numpy().astype(np.int64), x[batch].cpu().numpy().astype(np.int64),
+                                        idx))
+    got = c[0].double().cpu().numpy()[idx]
+    if dtype == "f64":
+        assert np.array_equal(np.rint(got).astype(np.int64), want)
+    else:
+        scale = 1024.0 ** 2 / 3 * np.sqrt(n)
+        assert np.abs(got - want).max() <= 3 * n_power * 2.0 ** -24 * 8 * scale
+
+
+@pytest.mark.parametrize("zero_pad", [False, True])
+@pytest.mark.parametrize("neg", [False, True])
+@pytest.mark.parametrize("n_power,batch,dtype,real", [
+    (12, 149, "f64", False), (12, 150, "f32", True), (12, 75, "f64", True), (13, 75, "f64", True),
+    (14, 38, "f32", False), (16, 10, "f64", False), (17, 5, "f32", False), (17, 5, "f64", True),
+    (18, 3, "f64", False)])
+def test_fft_tile_passes(gf, dev, n_power, batch, dtype, real, neg, zero_pad):
+    n = 1 << n_power
+    T = torch.float64 if dtype == "f64" else torch.float32
+    C = torch.complex128 if dtype == "f64" else torch.complex64
+    g = torch.Generator(device=dev).manual_seed(n_power * 1000 + batch)
+    if neg:  # X^N + 1: n entries e^(i pi (2 br(k) + 1) / 2^(s+1)) at [2^s, 2^(s+1))
+        import oracle
+        r, ri, _ = oracle.fft_tables(n, dtype)
+        roots, inv = torch.from_numpy(r).to(dev), torch.from_numpy(ri).to(dev)
+    else:
+        roots, inv = reference_table(gf, n, dtype, dev)
+    poly = gf.X_N_plus if neg else gf.X_N_minus
+    fwd = gf.fft_configuration(n_power=n_power, fft_type=gf.FORWARD, reduction_poly=poly, zero_padding=zero_pad)
+    bwd = gf.fft_configuration(n_power=n_power, fft_type=gf.INVERSE, reduction_poly=poly, mod_inverse=complex(1.0 / n))
+    x = torch.randn(2 * batch, n, device=dev, generator=g, dtype=T if real else C)
+
+    def product(rows, b):
+        if real:
+            temp = torch.empty(2 * b * n, dtype=C, device=dev)
+            out = torch.empty(b, n, dtype=T, device=dev)
+            gf.GPU_FFT(rows, temp, roots, fwd, 2 * b, False)
+            gf.GPU_FFT(out, temp, inv, bwd, b, True)
+            return out
+        buf = rows.clone()
+        gf.GPU_FFT(buf, roots, fwd, 2 * b, False)
+        gf.GPU_FFT(buf, inv, bwd, b, True)
+        return buf[:b]
+
+    c = product(x, batch)
+    few = product(torch.cat([x[batch - 1: batch], x[-1:]]), 1)
+    assert torch.equal(c[-1:], few)
+    u, v = x[:2].to(torch.complex128), x[batch:batch + 2].to(torch.complex128)
+    if zero_pad:
+        u[:, n // 2:] = 0
+        v[:, n // 2:] = 0
+    w = torch.exp(1j * np.pi / n * torch.arange(n, device=dev, dtype=torch.float64)) if neg else 1.0
+    want = torch.fft.ifft(torch.fft.fft(u * w) * torch.fft.fft(v * w)) / w
+    want = want.real if real else want
+    err = (torch.linalg.norm(c[:2].to(want.dtype) - want) / torch.linalg.norm(want)).item()
+    assert err < (1e-12 if dtype == "f64" else 2e-5)
