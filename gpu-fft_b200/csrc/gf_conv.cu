@@ -18,7 +18,7 @@
 //                contiguous middle pass (tile_product_kernel, TILE_VJP, from two
 //                2048-point tiles per SM on; vjp_kernel<12, false> below that),
 //                strided last inverse pass keeping the real parts (OUT_RE2).
-#include "gf_tile.cuh"
+#include "gf_single.cuh"
 
 namespace gfb
 {
@@ -168,6 +168,31 @@ static int linear_vjp(const float* g, const float* a, const float* b, float* ga,
         A.geo = PassGeo{};
         A.geo.m = m;
         const long long ctas = ((long long)batch * M + ECTA - 1) / ECTA;
+        // the one-kernel form writes grad_a before it reads a, and reads g and b of
+        // the next tile before that: results over operands take vjp_kernel, which
+        // holds all three operands first
+        const size_t row = (size_t)batch * M * sizeof(float);
+        auto clear = [](const float* x, size_t xb, const float* y, size_t yb) {
+            const char *px = reinterpret_cast<const char*>(x), *py = reinterpret_cast<const char*>(y);
+            return px + xb <= py || py + yb <= px;
+        };
+        bool apart = true;
+        for (float* o : {ga, gb}) apart = apart && clear(o, row, g, 2 * row) && clear(o, row, a, row) && clear(o, row, b, row);
+        if (m >= 4 && apart)
+        {
+            SingleArgs<float> k{};
+            k.park = g;
+            k.op[0] = b;
+            k.op[1] = a;
+            k.out[0] = ga;
+            k.out[1] = gb;
+            k.roots = A.roots;
+            k.twist = A.twist;
+            k.untwist = A.untwist;
+            k.scale = A.scale;
+            k.batch = batch;
+            return launch_single<float>(SINGLE_VJP, m, k, s);
+        }
         return dispatch_int<1, EBITS>(m, [&]<int LL>() { return launch_vjp_shape<LL, true>(A, ctas, s); });
     }
     long long W = vjp_wave(m, batch);

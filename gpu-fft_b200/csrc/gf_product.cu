@@ -21,7 +21,7 @@
 // sincospi in double precision (then rounded to float for the f32 path).
 #include "gf_fused.cuh"
 #include "gf_fused_r8.cuh"
-#include "gf_tile.cuh"
+#include "gf_single.cuh"
 
 #include <atomic>
 
@@ -164,7 +164,20 @@ template <typename T, bool SINGLE> static int launch_fused(const FusedArgs<T>& a
         }
         return launch_cluster_pass<T, CLM_FUSED>(c, a.batch, a.batch, s, a.geo.m);
     }
-    return dispatch_int<1, EBITS>(a.geo.m, [&]<int LL>() { return launch_fused_shape<T, LL, true>(a, ctas, s); });
+    if (a.geo.m >= 4)
+    {
+        SingleArgs<T> k{};
+        k.park = a.b;
+        k.op[0] = a.a;
+        k.out[0] = a.c;
+        k.roots = a.roots;
+        k.twist = a.twist;
+        k.untwist = a.untwist;
+        k.scale = a.scale;
+        k.batch = a.batch;
+        return launch_single<T>(a.cplx ? SINGLE_CYC : a.lin ? SINGLE_LIN : SINGLE_NEG, a.geo.m, k, s);
+    }
+    return dispatch_int<1, 3>(a.geo.m, [&]<int LL>() { return launch_fused_shape<T, LL, true>(a, ctas, s); });
 }
 
 // Pass plan of a wave of w products with 2^m-point transforms (m > 12): the

@@ -156,3 +156,43 @@ def test_fft_tile_passes(gf, dev, n_power, batch, dtype, real, neg, zero_pad):
     want = want.real if real else want
     err = (torch.linalg.norm(c[:2].to(want.dtype) - want) / torch.linalg.norm(want)).item()
     assert err < (1e-12 if dtype == "f64" else 2e-5)
+
+
+# one-kernel products (gf_single.cuh): 2^(11-m) to a tile, ragged last tiles, fewer
+# tiles than CTAs, several tiles per CTA
+@pytest.mark.parametrize("n_power,batch", [
+    (5, 1), (5, 127), (5, 129), (6, 33), (8, 5000), (9, 7), (10, 3), (10, 2501), (11, 65), (12, 67), (12, 601),
+    (13, 66), (13, 300)])
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+def test_single_products(gf, dev, n_power, batch, dtype):
+    n = 1 << n_power
+    T, C = (torch.float64, torch.complex128) if dtype == "f64" else (torch.float32, torch.complex64)
+    tol = (1e-14 if dtype == "f64" else 2e-6) * (n_power + 1)
+    g = torch.Generator(device=dev).manual_seed(n_power * 1000 + batch)
+
+    def err(got, want):
+        return (torch.linalg.norm(got.to(want.dtype) - want) / torch.linalg.norm(want)).item()
+
+    a, b = torch.randn(2, batch, n, device=dev, generator=g, dtype=T)
+    w = torch.exp(1j * np.pi / n * torch.arange(n, device=dev, dtype=torch.float64))
+    want = (torch.fft.ifft(torch.fft.fft(a.double() * w) * torch.fft.fft(b.double() * w)) / w).real
+    c = gf.negacyclic_mul(a, b)
+    assert err(c, want) < tol
+    inplace = a.clone()
+    assert torch.equal(gf.negacyclic_mul(inplace, b, out=inplace), c)
+    A, B = torch.fft.rfft(a.double(), 2 * n), torch.fft.rfft(b.double(), 2 * n)
+    if n_power <= 12:
+        assert err(gf.linear_mul(a, b), torch.fft.irfft(A * B, 2 * n)) < tol
+        x, y = torch.complex(a, b), torch.complex(b, a)
+        want = torch.fft.ifft(torch.fft.fft(x.to(torch.complex128)) * torch.fft.fft(y.to(torch.complex128)))
+        assert err(gf.cyclic_mul(x, y), want) < tol
+    if n_power <= 12 and dtype == "f32":
+        up = torch.randn(batch, 2 * n, device=dev, generator=g)
+        ga, gb = gf.linear_mul_vjp(up, a, b)
+        G = torch.fft.rfft(up.double(), 4 * n)
+        for got, z in ((ga, b), (gb, a)):
+            w4 = torch.fft.irfft(G * torch.fft.rfft(z.double(), 4 * n).conj(), 4 * n)[:, :n]
+            assert err(got, w4) < tol
+        a2, b2 = a.clone(), b.clone()  # results over the operands
+        gf.linear_mul_vjp(up, a2, b2, grad_a=a2, grad_b=b2)
+        assert torch.equal(a2, ga) and torch.equal(b2, gb)
