@@ -17,12 +17,19 @@
 // 16 consecutive points, stages 2048-point runs through padded shared memory
 // so that its global loads and stores stay coalesced too.
 //
+// From one 2048-point tile per SM on, the eleven or twelve smallest spans run as one
+// pass on tiles (special_tile_kernel), so that 2^15 points take two passes instead of
+// four.
+//
 // Launches with few 4096-point tiles (small batches, vectors of >= 4096
 // points) instead run the twelve smallest spans of every aligned tile as one
 // pass on an 8-CTA thread-block cluster (the layouts and DSMEM exchange of
 // gf_cluster.cuh): span 2^q of the tile is e-bit q, and its twiddle depends on
 // the bits below q, table[2^q + (e mod 2^q)].
 #include "gf_cluster.cuh"
+#include "gf_tile.cuh"
+
+#include <algorithm>
 
 namespace gfb
 {
@@ -80,7 +87,9 @@ __device__ __forceinline__ void special_network(cx<T> (&x)[1 << L], const cx<T> 
     }
 }
 
-// A pass of spans 2^p0 .. 2^(p0+L-1) (p0 > 0), one column per thread.
+// A pass of spans 2^p0 .. 2^(p0+L-1) (p0 > 0), one column per thread, in the vectors
+// blockIdx.y, blockIdx.y + gridDim.y, ...: a column's twiddles are its own (as many
+// bytes as its points) but the same in every vector.
 template <typename T, int L, bool FWD>
 __global__ void __launch_bounds__(SPECIAL_THREADS) special_col_kernel(const SpecialArgs<T> a)
 {
@@ -89,19 +98,22 @@ __global__ void __launch_bounds__(SPECIAL_THREADS) special_col_kernel(const Spec
     const long long idx = (long long)blockIdx.x * SPECIAL_THREADS + threadIdx.x;
     const int m = a.m, p0 = a.p0;
     const long long lo = idx & ((1LL << p0) - 1);
-    const long long rest = idx >> p0;
-    const long long hi = rest & ((1LL << (m - p0 - L)) - 1);
-    const long long b = rest >> (m - p0 - L);
-    if (b >= a.batch) return;
-    cx<T>* p = a.data + (b << m) + (hi << (p0 + L)) + lo;
+    const long long hi = idx >> p0;
+    if (hi >= (1LL << (m - p0 - L))) return;
+    cx<T>* p = a.data + (hi << (p0 + L)) + lo;
     cx<T> w[R - 1];
     special_twiddles<T, L>(w, a, lo);
-    cx<T> x[R];
+#pragma unroll 1
+    for (long long b = blockIdx.y; b < a.batch; b += gridDim.y)
+    {
+        cx<T>* q = p + (b << m);
+        cx<T> x[R];
 #pragma unroll
-    for (int k = 0; k < R; k++) x[k] = p[(long long)k << p0];
-    special_network<T, L, FWD>(x, w, a);
+        for (int k = 0; k < R; k++) x[k] = q[(long long)k << p0];
+        special_network<T, L, FWD>(x, w, a);
 #pragma unroll
-    for (int k = 0; k < R; k++) p[(long long)k << p0] = x[k];
+        for (int k = 0; k < R; k++) q[(long long)k << p0] = x[k];
+    }
 }
 
 // The pass of the smallest spans (p0 = 0): every column is 2^L consecutive
@@ -256,6 +268,103 @@ __global__ void __cluster_dims__(CL_CTAS, 1, 1) __launch_bounds__(CL_THREADS) sp
     }
 }
 
+// Radix-16 round of the special network on the e-bits [W, W + HI) held by the
+// register bits [0, HI): the lower point of a pair at e-bit W + i uses
+// table[2^(W+i) + (lo + ((r mod 2^i) << W))], lo the thread's e-bits below W.
+template <typename T, bool FWD, int W, int HI>
+__device__ __forceinline__ void special_round(cx<T> (&x)[16], int lo, const cx<T>* __restrict__ tab)
+{
+#pragma unroll
+    for (int k = 0; k < HI; k++)
+    {
+        const int i = FWD ? k : HI - 1 - k;
+        cx<T> w[8];
+#pragma unroll
+        for (int h = 0; h < 8; h++)
+            if (h < (1 << i)) w[h] = ldg<T>(tab + (1 << (W + i)) + lo + (h << W));
+#pragma unroll
+        for (int r = 0; r < 16; r++)
+        {
+            if (r & (1 << i)) continue;
+            const cx<T> wt = w[r & ((1 << i) - 1)];
+            if (FWD)
+                ct_bfly<T>(x[r], x[r | (1 << i)], wt);
+            else
+                gs_bfly<T>(x[r], x[r | (1 << i)], wt);
+        }
+    }
+}
+
+// Spans 2^0 .. 2^(LT-1) of every aligned 2^LT-point tile (vectors of 2^m >= 2^LT
+// points) in one pass on 2^LT / 16 threads (the layouts and transposes of TileOf).
+// The twiddles depend on the position in the tile only: every CTA reads the same
+// 2^LT table entries, coalesced (the outer round) or the same for many threads, from
+// L1. Three passes of four spans become one (2^15 points, 65 vectors, FP64, a
+// direction: 49 -> 20 us; encode and decode with their copies 109 -> 72).
+template <typename T, bool FWD, int LT>
+__global__ void __launch_bounds__(TileOf<LT>::HT, (sizeof(T) == 8 ? 4 : 6) / (LT - 10)) special_tile_kernel(const SpecialArgs<T> a)
+{
+    pdl_begin(); // before any global-memory access (programmatic launch)
+    using tl = TileOf<LT>;
+    constexpr int R = 16, HT = tl::HT;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cx<T>* sm = reinterpret_cast<cx<T>*>(smraw);
+    const int t = threadIdx.x;
+    cx<T>* p = a.data + ((long long)blockIdx.x << LT) + t;
+    cx<T> x[16];
+#pragma unroll
+    for (int r = 0; r < R; r++) x[r] = p[r * HT];
+    if constexpr (FWD)
+    {
+        tl::template put<tl::W1>(x, sm, t);
+        __syncthreads();
+        tl::template get<0>(x, sm, t);
+        special_round<T, true, 0, tl::HI0>(x, 0, a.table);
+        tl::template put<0>(x, sm, t);
+        __syncthreads();
+        tl::template get<tl::W2>(x, sm, t);
+        special_round<T, true, tl::W2, 4>(x, t & ((1 << tl::W2) - 1), a.table);
+        tl::template put<tl::W2>(x, sm, t);
+        __syncthreads();
+        tl::template get<tl::W1>(x, sm, t);
+        special_round<T, true, tl::W1, 4>(x, t, a.table);
+    }
+    else
+    {
+        special_round<T, false, tl::W1, 4>(x, t, a.table);
+        tl::template put<tl::W1>(x, sm, t);
+        __syncthreads();
+        tl::template get<tl::W2>(x, sm, t);
+        special_round<T, false, tl::W2, 4>(x, t & ((1 << tl::W2) - 1), a.table);
+        tl::template put<tl::W2>(x, sm, t);
+        __syncthreads();
+        tl::template get<0>(x, sm, t);
+        special_round<T, false, 0, tl::HI0>(x, 0, a.table);
+        tl::template put<0>(x, sm, t);
+        __syncthreads();
+        tl::template get<tl::W1>(x, sm, t);
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) p[r * HT] = a.do_scale ? cmul<T>(x[r], a.scale) : x[r];
+}
+
+template <typename T, bool FWD, int LT> static int launch_special_tile_lt(const SpecialArgs<T>& a, cudaStream_t s)
+{
+    static int done[64] = {0};
+    const size_t smem = (size_t)TileOf<LT>::SLOT * sizeof(cx<T>);
+    const int st = ensure_smem(special_tile_kernel<T, FWD, LT>, smem, done);
+    if (st) return st;
+    const long long tiles = (a.batch << a.m) >> LT;
+    if (tiles > 0x7fffffffLL) return GPUFFT_ERROR_INVALID_VALUE;
+    GF_TRACE(tr, (double)(a.batch << a.m) * 2 * sizeof(cx<T>), s, "special_tile<%s,%s,L%d>", sizeof(T) == 4 ? "f32" : "f64",
+             FWD ? "fwd" : "inv", LT);
+    return launch_k(special_tile_kernel<T, FWD, LT>, dim3((unsigned)tiles), dim3(TileOf<LT>::HT), smem, s, a);
+}
+template <typename T, bool FWD> static int launch_special_tile(const SpecialArgs<T>& a, int LT, cudaStream_t s)
+{
+    return LT == 11 ? launch_special_tile_lt<T, FWD, 11>(a, s) : launch_special_tile_lt<T, FWD, 12>(a, s);
+}
+
 template <typename T, bool FWD> static int launch_special_cluster(const SpecialArgs<T>& a, cudaStream_t s)
 {
     const long long tiles = (a.batch << a.m) >> EBITS;
@@ -276,10 +385,13 @@ template <typename T, bool FWD> static int launch_special_pass(const SpecialArgs
             return launch_k(special_first_kernel<T, LL, FWD>, dim3((unsigned)((points + RUN - 1) / RUN)),
                             dim3(SPECIAL_THREADS), 0, s, a);
         }
-        const long long threads = points >> LL;
-        return launch_k(special_col_kernel<T, LL, FWD>,
-                        dim3((unsigned)((threads + SPECIAL_THREADS - 1) / SPECIAL_THREADS)), dim3(SPECIAL_THREADS), 0,
-                        s, a);
+        // vectors per thread: as many as leave two CTAs' worth of columns per slot
+        // (three CTAs per SM in FP64, five in FP32)
+        const long long bx = ((1LL << (a.m - LL)) + SPECIAL_THREADS - 1) / SPECIAL_THREADS;
+        const long long want = (long long)sm_count() * (sizeof(T) == 8 ? 6 : 10);
+        const long long per = std::min<long long>(8, std::max<long long>(1, bx * a.batch / want));
+        const long long by = std::min<long long>(65535, (a.batch + per - 1) / per);
+        return launch_k(special_col_kernel<T, LL, FWD>, dim3((unsigned)bx, (unsigned)by), dim3(SPECIAL_THREADS), 0, s, a);
     });
 }
 
@@ -291,14 +403,19 @@ static int special_fft(cx<T>* inout, const cx<T>* table, int n_power, int fft_ty
     if (!inout || !table || batch <= 0 || (fft_type != GPUFFT_FORWARD && fft_type != GPUFFT_INVERSE))
         return GPUFFT_ERROR_INVALID_VALUE;
     if ((uintptr_t)inout % sizeof(cx<T>) || (uintptr_t)table % sizeof(cx<T>)) return GPUFFT_ERROR_MISALIGNED;
-    // few tiles: the twelve smallest spans as one cluster pass (L = 12 below)
+    // few tiles: the twelve smallest spans as one cluster pass. Otherwise, from one
+    // 2048-point tile per SM on, the eleven or twelve smallest as one tile pass:
+    // twelve where that saves a pass of the rest.
     const long long tiles = ((long long)batch << n_power) >> EBITS;
     const bool cl = n_power >= EBITS && cluster_ok(tiles);
+    const int first = cl ? EBITS
+                      : n_power >= 11 && 2 * tiles >= sm_count() ? (n_power % 4 == 0 ? 12 : 11)
+                                                                 : 4;
     int p0s[8], Ls[8], np = 0;
-    for (int p0 = 0; p0 < n_power; p0 += (cl && p0 == 0) ? EBITS : 4)
+    for (int p0 = 0; p0 < n_power; p0 += p0 == 0 ? first : 4)
     {
         p0s[np] = p0;
-        Ls[np] = (cl && p0 == 0) ? EBITS : ((n_power - p0) < 4 ? (n_power - p0) : 4);
+        Ls[np] = p0 == 0 && first > 4 ? first : ((n_power - p0) < 4 ? (n_power - p0) : 4);
         np++;
     }
     SpecialArgs<T> a{};
@@ -313,7 +430,10 @@ static int special_fft(cx<T>* inout, const cx<T>* table, int n_power, int fft_ty
         a.p0 = p0s[k];
         a.do_scale = fft_type == GPUFFT_INVERSE && i == np - 1;
         int st;
-        if (Ls[k] == EBITS)
+        if (Ls[k] > 4 && !cl)
+            st = fft_type == GPUFFT_FORWARD ? launch_special_tile<T, true>(a, Ls[k], s)
+                                            : launch_special_tile<T, false>(a, Ls[k], s);
+        else if (Ls[k] == EBITS)
             st = fft_type == GPUFFT_FORWARD ? launch_special_cluster<T, true>(a, s)
                                             : launch_special_cluster<T, false>(a, s);
         else

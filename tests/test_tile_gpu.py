@@ -196,3 +196,27 @@ def test_single_products(gf, dev, n_power, batch, dtype):
         a2, b2 = a.clone(), b.clone()  # results over the operands
         gf.linear_mul_vjp(up, a2, b2, grad_a=a2, grad_b=b2)
         assert torch.equal(a2, ga) and torch.equal(b2, gb)
+
+
+# the tile pass of the smallest spans: from 148 2048-point tiles on
+@pytest.mark.parametrize("n_power,batch", [(11, 148), (11, 149), (12, 75), (13, 38), (14, 19), (15, 10), (16, 5), (17, 9),
+                                           (20, 2)])
+@pytest.mark.parametrize("C", [torch.complex128, torch.complex64])
+def test_special_tile_rows(gf, O, dev, n_power, batch, C):
+    n = 1 << n_power
+    g = torch.Generator(device=dev).manual_seed(n_power * 100 + batch)
+    x = torch.randn(batch, n, device=dev, generator=g, dtype=C)
+    tab = torch.polar(torch.ones(n, device=dev, dtype=torch.float64),
+                      torch.rand(n, device=dev, generator=g, dtype=torch.float64) * 6.283185307179586).to(C)
+    mi = complex(1.0 / n, 0.5 / n)
+    for kind in (gf.FORWARD, gf.INVERSE):
+        cfg = gf.fft_configuration(n_power=n_power, fft_type=kind, mod_inverse=mi)
+        y, few = x.clone(), x[-1:].clone()
+        gf.GPU_Special_FFT(y, tab, cfg, batch)
+        gf.GPU_Special_FFT(few, tab, cfg, 1)
+        assert torch.equal(y[-1:], few)
+        if n_power <= 16:
+            np_c = np.complex128 if C == torch.complex128 else np.complex64
+            want = O.gpu_special_fft(x[0].cpu().numpy().astype(np_c), tab.cpu().numpy(), n_power, kind, mi, 1)
+            err = np.linalg.norm(y[0].cpu().numpy() - want.ravel()) / np.linalg.norm(want)
+            assert err < (1e-12 if C == torch.complex128 else 2e-5)
