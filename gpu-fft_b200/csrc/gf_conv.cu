@@ -134,7 +134,7 @@ static long long vjp_wave(int m, long long batch)
     // tile kernel's rings (512 rows of N = 2^14, all kernels of the call: four
     // waves of 128 with the 4096-point middle pass 368 us, one with the tile kernel 187 us)
     const size_t per = 3 * ((size_t)1 << m) * sizeof(cx<float>);
-    long long w = (long long)((m - TILE_LT <= COL_MAX_L ? 320ull << 20 : 48ull << 20) / per);
+    long long w = (long long)((m - TILE_LT <= TILE_MAX_L ? 320ull << 20 : 48ull << 20) / per);
     if (w < 1) w = 1;
     return w < batch ? w : batch;
 }
@@ -204,7 +204,7 @@ static int linear_vjp(const float* g, const float* a, const float* b, float* ga,
     {
         const long long w = (batch - p0) < W ? (batch - p0) : W;
         Plan p = make_plan(m);
-        const bool tiled = m - TILE_LT <= COL_MAX_L && (w << (m - TILE_LT)) >= 2LL * sm_count();
+        const bool tiled = m - TILE_LT <= TILE_MAX_L && (w << (m - TILE_LT)) >= 2LL * sm_count();
         if (tiled)
         {
             p.L[0] = m - TILE_LT;

@@ -187,7 +187,7 @@ template <typename T, bool SINGLE> static int launch_fused(const FusedArgs<T>& a
 template <typename T> static Plan product_plan(int m, long long w)
 {
     Plan p = make_plan(m);
-    if (m - TILE_LT > COL_MAX_L || (w << (m - TILE_LT)) < 2LL * sm_count()) return p;
+    if (m - TILE_LT > TILE_MAX_L || (w << (m - TILE_LT)) < 2LL * sm_count()) return p;
     if (sizeof(T) == 8 && !g_f64_middle_r8.load(std::memory_order_relaxed)) return p;
     p.L[0] = m - TILE_LT;
     p.L[1] = TILE_LT;
@@ -229,7 +229,7 @@ static long long wave_products(int n_power, long long batch, size_t cx_bytes)
     const int m = n_power - 1;
     if (m <= EBITS) return batch;
     const size_t per = 2 * ((size_t)1 << m) * cx_bytes;
-    long long w = (long long)((m - TILE_LT <= COL_MAX_L ? WAVE_TILE_BYTES : WAVE_TARGET_BYTES) / per);
+    long long w = (long long)((m - TILE_LT <= TILE_MAX_L ? WAVE_TILE_BYTES : WAVE_TARGET_BYTES) / per);
     if (w < 1) w = 1;
     w = round_wave(w, ((long long)1 << m) / ECTA);
     return w < batch ? w : batch;

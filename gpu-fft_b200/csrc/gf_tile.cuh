@@ -228,6 +228,9 @@ template <int LT> struct TileOf
     }
 };
 constexpr int TILE_LT = 11;
+// most stages left for the pass before the tiles (a column pass up to COL_MAX_L, a
+// strided pass of 4096-point tiles above)
+constexpr int TILE_MAX_L = 9;
 using tile = TileOf<TILE_LT>;
 
 enum TileMode
