@@ -178,10 +178,19 @@ class fft_configuration:
     stream: Optional[object] = None  # torch.cuda.Stream, a raw cudaStream_t int, or None
 
 
+def _current_stream_raw() -> int:
+    """The current stream's cudaStream_t. torch's raw getter takes 0.4 us; building a
+    Stream object for torch.cuda.current_stream() takes 3.4, a third of a small call."""
+    import torch
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None:
+        return torch.cuda.current_stream().cuda_stream
+    return raw(torch.cuda.current_device())
+
+
 def _stream_handle(stream) -> Optional[int]:
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream or None
+        return _current_stream_raw() or None
     if isinstance(stream, int):
         return stream or None
     return stream.cuda_stream or None
