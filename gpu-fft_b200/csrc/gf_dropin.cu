@@ -9,16 +9,18 @@
 //     21 < m <= 24   passes of (m-21, 9, 12) stages
 // where m = log2 of the transform length (n_power for GPU_FFT, n_power-1 for
 // GPU_FFNT). Reference: src/lib/fft.cu:517-725 (GPU_FFT), 1386-1515 (GPU_FFNT).
-#include "gf_pass.cuh"
+#include "gf_tile.cuh"
 
 #include <cstdio>
 
 namespace gfb
 {
 
-// Passes of (m - 11, 11) stages, the second on 2048-point tiles, where the column
-// pass has a kernel for the rest and two tiles per SM keep the tile pass's CTAs
-// overlapping; the plan above otherwise. FP64 FFNT calls (fold) keep 4096-point
+// Passes of (m - 11, 11) stages, the second on 2048-point tiles, where a column pass
+// (FP64, up to 2^16 points) or any first pass (FP32, up to 2^20: C_C N = 2^20, batch
+// 11, 319 us against 353; FP64 328 against 306 at batch 5) has a kernel for the rest
+// and two tiles per SM keep the tile pass's CTAs overlapping; the plan above
+// otherwise. FP64 FFNT calls (fold) keep 4096-point
 // tiles from three per two SMs on: one column stage fewer next to the fold, longer
 // runs under one staging of the twiddles (product, N = 2^16: batch 256 351 against
 // 413 us, batch 30 52 against 59; N = 2^15, batch 20, below the line: 36 against 34;
@@ -26,7 +28,8 @@ namespace gfb
 template <typename T> static Plan transform_plan(int m, long long batch, bool fold)
 {
     Plan p = make_plan(m);
-    if (m <= EBITS || m - 11 > COL_MAX_L || (batch << (m - 11)) < 2LL * sm_count()) return p;
+    if (m <= EBITS || m - 11 > (sizeof(T) == 4 ? TILE_MAX_L : COL_MAX_L) || (batch << (m - 11)) < 2LL * sm_count())
+        return p;
     if (sizeof(T) == 8 && fold && 2 * (batch << (m - EBITS)) >= 3LL * sm_count()) return p;
     p.L[0] = m - 11;
     p.L[1] = 11;

@@ -115,7 +115,7 @@ def test_ffnt_tile_passes(gf, O, dev, n_power, batch, dtype):
 @pytest.mark.parametrize("n_power,batch,dtype,real", [
     (12, 149, "f64", False), (12, 150, "f32", True), (12, 75, "f64", True), (13, 75, "f64", True),
     (14, 38, "f32", False), (16, 10, "f64", False), (17, 5, "f32", False), (17, 5, "f64", True),
-    (18, 3, "f64", False)])
+    (18, 3, "f64", False), (19, 2, "f32", False), (20, 2, "f32", True)])
 def test_fft_tile_passes(gf, dev, n_power, batch, dtype, real, neg, zero_pad):
     n = 1 << n_power
     T = torch.float64 if dtype == "f64" else torch.float32
