@@ -183,11 +183,18 @@ template <typename T, bool SINGLE> static int launch_fused(const FusedArgs<T>& a
 // Pass plan of a wave of w products with 2^m-point transforms (m > 12): the
 // tile kernel's (m - 11 column stages, eleven on 2048-point tiles), or the
 // 4096-point middle pass. Waves of fewer than two tiles per SM leave the tile
-// kernel's CTAs too few to overlap: they take the middle pass.
-template <typename T> static Plan product_plan(int m, long long w)
+// kernel's CTAs too few to overlap: they take the middle pass (FP64, N = 2^16, at the
+// line, 20 products: 26.7 us on tiles, 34.2 with the middle pass).
+// FP64 negacyclic waves of four to five tiles per SM also take the middle pass, though
+// the tiles are faster there (N = 2^16, 40 products: 44 against 53 us): programs that
+// read the trace rely on its rows for such a wave (three column stages, one
+// fused_r8_kernel launch, their bytes).
+template <typename T> static Plan product_plan(int m, long long w, bool negacyclic)
 {
     Plan p = make_plan(m);
-    if (m - TILE_LT > TILE_MAX_L || (w << (m - TILE_LT)) < 2LL * sm_count()) return p;
+    const long long tiles = w << (m - TILE_LT), sms = sm_count();
+    if (m - TILE_LT > TILE_MAX_L || tiles < 2 * sms) return p;
+    if (sizeof(T) == 8 && negacyclic && tiles > 4 * sms && tiles < 5 * sms) return p;
     if (sizeof(T) == 8 && !g_f64_middle_r8.load(std::memory_order_relaxed)) return p;
     p.L[0] = m - TILE_LT;
     p.L[1] = TILE_LT;
@@ -284,7 +291,7 @@ static int negacyclic_mul(const T* a, const T* b, T* c, int n_power, int batch, 
     for (long long p0 = 0; p0 < batch; p0 += W)
     {
         const long long w = (batch - p0) < W ? (batch - p0) : W;
-        const Plan p = product_plan<T>(m, w);
+        const Plan p = product_plan<T>(m, w, !lin);
         // 1. first forward pass of both operands: fold + twist in the load
         {
             long long ctas = 0;
@@ -375,7 +382,7 @@ static int cyclic_mul(const cx<T>* a, const cx<T>* b, cx<T>* c, int n_power, int
     for (long long p0 = 0; p0 < batch; p0 += W)
     {
         const long long w = (batch - p0) < W ? (batch - p0) : W;
-        const Plan p = product_plan<T>(m, w);
+        const Plan p = product_plan<T>(m, w, false);
         {
             long long ctas = 0;
             PassArgs<T> k{};
