@@ -313,6 +313,11 @@ template <int K> __global__ void __launch_bounds__(tile::HT, tile_min_blocks<dou
     const long long base = ((long long)blockIdx.x << 11) + t; // flat over the products
     const long long g = (long long)blockIdx.x & ((1LL << (m - 11)) - 1);
     const long long WM = a.W * M;
+    if (t == 0) // the other limbs wait in L2 (N = 2^16, batch 256, 24 bits: 437 -> 431 us)
+    {
+#pragma unroll
+        for (int l = 1; l < K; l++) prefetch_l2(a.spec + l * WM + base, tile::P * sizeof(cx<double>));
+    }
     cx<double> pk[R], x[R];
 #pragma unroll
     for (int r = 0; r < R; r++) pk[r] = a.spec[K * WM + base + (r << 7)];

@@ -9,8 +9,9 @@
 // many shared-memory cycles as the data's whole way through the pass). The tile's
 // index T selects its twiddles, so the CTAs are persistent, each with a run of
 // (T, row) pairs in T-major order: the twiddles are staged once for many rows.
-// While a tile is transformed the next one's loads are in flight (not for products,
-// whose two operands of two tiles do not fit the registers).
+// While a tile is transformed the next one's loads are in flight; for products, whose
+// two operands of two tiles do not fit the registers, the next tile's rows are asked
+// for in L2 (FFNT product FP64, N = 2^16, batch 256: 360 -> 354 us).
 //
 // FP64 forward tiles leave through the TMA unit: after its last round a thread holds
 // 16 consecutive points, writes them to its own 256 bytes of the padded buffer and
@@ -220,6 +221,12 @@ __global__ void __launch_bounds__(TilePass<LT>::HT, tile_pass_blocks<T, LT>())
         }
         else
         {
+            if (t == 0 && u + 1 < u1)
+            {
+                const cx<T>* p = reinterpret_cast<const cx<T>*>(a.in) + row * M + (g << LT);
+                prefetch_l2(p, tl::P * sizeof(cx<T>));
+                prefetch_l2(p + a.prod_off, tl::P * sizeof(cx<T>));
+            }
             tile_load<T, LT, IK>(a, x, gc, b, t);
         }
         if constexpr (IK == IN_FOLD)
