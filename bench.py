@@ -600,8 +600,13 @@ def time_path(step, host_step, a, b, c, hosts, args, stream, torch, barrier, max
 # replay, so this is the cold-cache figure). Both scale with the products per
 # launch, so traffic per launch = ratio x the kernel's tagged bytes per launch.
 NCU_TRAFFIC = {
-    # 64 products (1024 tiles): 168.8 MB read + 99.8 MB written of 318.8 MB tagged
-    "split_tile<k5>": (268.5 / 318.8, "ncu capture of a 64-product launch"),
+    # 128 products (2048 tiles of 2048 points), DRAM rate x duration of the capture:
+    # 281.6 MB of 335.5 MB tagged
+    "split_tile<f64,k2>": (281.6 / 335.5, "ncu capture of a 128-product launch"),
+    # 157.3 MB of 201.3 MB tagged
+    "tile_product<f64,mul>": (157.3 / 201.3, "ncu capture of a 128-product launch"),
+    # 211.5 MB of 268.4 MB tagged
+    "tile_pass<f64,fwd,L12,in0,out0>": (211.5 / 268.4, "ncu capture of a 128-product launch"),
     # wave of 74 products (592 tiles): 78.1 MB read + 2.7 MB written of 116.4 MB tagged
     "fused_r8_kernel<f64,L12,middle>": (80.9 / 116.4, "ncu capture of a 74-product wave"),
     # wave of 46 products (3680 CTAs): 120.8 MB read + 63.5 MB written of 241.2 MB tagged
