@@ -378,7 +378,7 @@ def negacyclic_mul_split(a, b, out=None, input_bits=None, non_negative=None, lim
     FP32 (precision="f32", N <= 2^22, float tables) or FP64 (precision="f64", N <= 2^17,
     double tables) transforms; returns an int64 tensor (and the max pre-rounding error).
     Plans within the error model run on FP64 transforms with b whole where that is
-    faster (include/gpufft_b200.h); the integers are the same."""
+    faster (include/gpufft_b200.h), which also holds rows whose coefficients add up."""
     import torch
     batch, n = a.shape
     n_power = n.bit_length() - 1
@@ -422,7 +422,8 @@ def set_f64_middle(r8: int) -> int:
 def set_split_tile(on: int) -> int:
     """Exact products run on FP64 transforms with one operand whole (1, the
     default) or as the chain of limb passes (0); a negative value queries. The
-    integers are the same either way. Returns the previous setting."""
+    integers are the same wherever the chain reports an error below 0.5. Returns the
+    previous setting."""
     return int(lib().gpufft_set_split_tile(int(on)))
 
 

@@ -11,8 +11,8 @@
 namespace gfb
 {
 // Exact products run on FP64 transforms with one operand whole (split_exact; 1,
-// the default) or with both operands cut into the plan's limbs (0). Both give the
-// same integers; set by gpufft_set_split_tile.
+// the default) or with both operands cut into the plan's limbs (0), which holds
+// uniform rows but not every coherent one. Set by gpufft_set_split_tile.
 static std::atomic<int> g_split_tile{1};
 
 // --------------------------------------------------------------------------
@@ -173,8 +173,9 @@ static int split_mul(const int32_t* a, const int32_t* b, int64_t* c, int n_power
         cudaError_t e = cudaMemsetAsync(max_err, 0, sizeof(unsigned), s);
         if (e != cudaSuccess) return set_cuda_error(e);
     }
-    // a plan within the error model is exact, and so is split_exact; a plan chosen
-    // outside it runs as given, so that its error report is its own
+    // a plan within the error model holds uniform rows, and split_exact those and
+    // coherent ones; a plan chosen outside it runs as given, so that its error report
+    // is its own
     if (g_split_tile.load(std::memory_order_relaxed))
     {
         double mag = 0;
@@ -184,7 +185,7 @@ static int split_mul(const int32_t* a, const int32_t* b, int64_t* c, int n_power
         {
             const cx<double>* t64 = nullptr;
             if constexpr (!F32) t64 = tab;
-            const int st = split_exact(a, b, c, m, batch, input_bits, non_negative != 0, w, k, t64, ws, ws_bytes, max_err, s);
+            const int st = split_exact(a, b, c, m, batch, input_bits, non_negative != 0, t64, ws, ws_bytes, max_err, s);
             if (st >= 0) return st;
         }
     }

@@ -628,9 +628,9 @@ template <int L, bool SINGLE, int K> static int launch_mid_k(const SplitArgs& a,
 // The exact product on FP64 transforms (gf_split_tile.cuh), or -1 where it does
 // not apply (the caller then runs the limb plan): tables is the FP64 native block,
 // or null (FP32 callers): the call then makes its own twiddles in the workspace.
-// (plan_w, plan_k): the caller's limb plan, whose exactness is kept.
+// Its limbs follow the call's ring, width and sign, whatever the caller's plan.
 int split_exact(const int32_t* a, const int32_t* b, int64_t* c, int m, int batch, int input_bits, bool non_negative,
-                int plan_w, int plan_k, const cx<double>* tables, void* ws, size_t ws_bytes, unsigned* max_err, cudaStream_t s);
+                const cx<double>* tables, void* ws, size_t ws_bytes, unsigned* max_err, cudaStream_t s);
 
 // one-kernel products for rings N <= 8192 (transform length 2^L, L = 1..12),
 // compiled in separate translation units by L range

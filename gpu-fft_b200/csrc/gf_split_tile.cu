@@ -34,50 +34,57 @@ __global__ void exact_tables_kernel(cx<double>* tab, int m)
     }
 }
 
-// The fewest limbs K of a (width w) that hold both kinds of data:
+// The fewest limbs K of a (width w) that hold both kinds of data, for operands of
+// magnitude at most 2^B (after centring):
 //   - uniform: the error model of the equal-limb plans (7.1 rms rms sqrt(N)
 //     sqrt(log2(N/2)) 2^-53 per pair, pairs of a group in quadrature; measured at
 //     most 1.2 of it) predicts at most 0.06;
-//   - coherent (constant or zero rows, zero-padded ones): a group's coefficients
-//     reach N 2^(top + B) and their error about 2^-50 of that (N = 2^12, 24 bits:
-//     2^46 and 0.05; N = 2^14: 2^48 and 0.19), so that is kept at most `coherent`.
-// Magnitudes of both operands (after centring) are at most 2^B.
-static bool exact_plan(int n_power, int B, bool centred, double coherent, int* w_out, int* k_out)
+//   - coherent (constant, half-range or zero rows, zero-padded ones), whose
+//     coefficients add up: limb l's product reaches N 2^t 2^B (t: the limb's bits),
+//     with b' + C u of up to 2^(B+1) for centred calls, whose last limb also carries
+//     2^t U B'. The error such rows leave is at most 2^-50 of that bound (measured
+//     over rings 2^5 .. 2^17 and 8 to 30 bits, on constant, half-range, zero-padded,
+//     ramped and alternating rows: 0.3 .. 1.0 of 2^-50), so the bound may not pass
+//     2^48 (largest error seen 0.19; 24 bits at N = 2^16 take three limbs).
+// The bound does not depend on what the caller's own plan would hold.
+static bool exact_plan(int n_power, int B, bool centred, int* w_out, int* k_out)
 {
     const double rb = std::ldexp(1.0, B) / std::sqrt(3.0), cen = centred ? std::ldexp(1.0, B) : 0.0;
-    const double sqn = std::sqrt(std::ldexp(1.0, n_power));
+    const double model = 7.1 * std::sqrt(std::ldexp(1.0, n_power)) * std::sqrt((double)(n_power - 1)) * std::ldexp(1.0, -53);
     for (int K = 1; K <= EXACT_MAX_LIMBS; K++)
     {
-        double best = 0, coh = 0;
+        double best = 0;
         int bw = 0;
-        for (int w = 1; w <= 20; w++)
+        for (int w = 1; w <= (K > 1 ? 20 : 1); w++)
         {
             const int top = B - w * (K - 1);
-            if (K == 1 && w > 1) break;
             if (top < 0) continue;
-            double worst = 0;
+            double worst = 0, mag = 0;
             for (int l = 0; l < K; l++)
             {
-                const double ra = std::ldexp(1.0, l == K - 1 ? top : w - 1) / std::sqrt(3.0);
+                const bool last = l == K - 1;
+                const double da = std::ldexp(1.0, last ? top : w - 1), ra = da / std::sqrt(3.0);
                 double e2 = ra * ra * (rb * rb + cen * cen);
-                if (l == K - 1 && centred) e2 += rb * rb * std::ldexp(1.0, 2 * top);
+                double g = da * (std::ldexp(1.0, B) + cen);
+                if (last && centred)
+                {
+                    e2 += rb * rb * std::ldexp(1.0, 2 * top);
+                    g += std::ldexp(1.0, top + B);
+                }
                 worst = std::max(worst, std::sqrt(e2));
+                mag = std::max(mag, std::ldexp(g, n_power));
             }
+            if (model * worst > 0.06 || mag > std::ldexp(1.0, 48)) continue;
             if (bw == 0 || worst < best)
             {
                 best = worst;
                 bw = w;
-                coh = std::ldexp(1.0, n_power + std::max(top, K > 1 ? w - 1 : 0) + B);
             }
         }
         if (bw == 0) continue;
-        const double err = 7.1 * best * sqn * std::sqrt((double)(n_power - 1)) * std::ldexp(1.0, -53);
-        if (err <= 0.06 && coh <= coherent)
-        {
-            *w_out = bw;
-            *k_out = K;
-            return true;
-        }
+        *w_out = bw;
+        *k_out = K;
+        return true;
     }
     return false;
 }
@@ -122,22 +129,13 @@ template <int m, int K> static int launch_exact_single(const ExactArgs& a, cudaS
 }
 
 int split_exact(const int32_t* a, const int32_t* b, int64_t* c, int m, int batch, int input_bits, bool non_negative,
-                int plan_w, int plan_k, const cx<double>* tables, void* ws, size_t ws_bytes, unsigned* max_err, cudaStream_t s)
+                const cx<double>* tables, void* ws, size_t ws_bytes, unsigned* max_err, cudaStream_t s)
 {
     const long long M = 1LL << m;
     if (m < 4 || m > 16 || (reinterpret_cast<uintptr_t>(ws) & 15)) return -1;
-    // Coherent rows: an FP64 plan of several limbs holds them with little error, so
-    // such calls stay below 2^47 here, the others below 2^48. FP32 plans lose them
-    // where their top limbs' products pass 2^22 (reported as 1.0); there only the
-    // uniform model decides, up to the magnitudes measured to lose no more rows than
-    // the FP32 plan (zero rows of N = 2^16 and 24 bits are off, and reported, in both).
     const int B = non_negative ? input_bits - 1 : input_bits;
-    const int ptop = B - plan_w * (plan_k - 1);
-    int coherent = tables && plan_k > 1 ? 47 : 48;
-    if (!tables && m + 1 + (non_negative ? ptop + B % plan_w + 1 : 2 * ptop) >= (non_negative ? 23 : 22))
-        coherent = non_negative ? 50 : 52;
     int w = 0, K = 0;
-    if (!exact_plan(m + 1, B, non_negative, std::ldexp(1.0, coherent), &w, &K)) return -1;
+    if (!exact_plan(m + 1, B, non_negative, &w, &K)) return -1;
     const bool single = m <= 12;
     // one CTA runs its product's transforms in turn: few 4096-point ones take the
     // chain, which spreads them (one product of 24 bits: 24.6 against 31.2 us)

@@ -4,12 +4,15 @@
 // c = a b mod (X^N + 1) for integers |a_i|, |b_i| < 2^B. An FP64 transform pair
 // leaves an error of about 7 rms(a) rms(b) sqrt(N log2 N) 2^-53 per coefficient
 // (the model of gf_split.cu): at B = 23 and N = 2^16 that is 18, far above 0.5, but
-// with a alone cut into K = 2 limbs of 12 bits it is 0.005. So a is cut into the
-// fewest limbs (one up to about 18 bits, two at 24) and b stays whole: K + 1
-// forward and K inverse FP64 transforms, where equal FP32 limbs of both operands
-// take 4k - 1 (19 for 24 bits) and equal FP64 limbs 4K - 1. B200 runs FP64 at half
-// the FP32 rate, so 5 against 19 is a quarter of the arithmetic, and the spectra
-// in memory fall from 19 x 8 to 3 x 16 bytes per point. The integers are the same.
+// with a alone cut into K = 2 limbs of 12 bits it is 0.005. Rows whose coefficients
+// add up need more: a limb's product of N 2^11 2^23 or three times that is beyond
+// what a double holds to 0.5, and three limbs of 8 bits keep it below 2^48
+// (exact_plan). So a is cut into the fewest limbs that hold every row of the call
+// (one up to 16 bits, three at 24 bits and N = 2^16) and b stays whole: K + 1 forward
+// and K inverse FP64 transforms, where equal FP32 limbs of both operands take 4k - 1
+// (19 for 24 bits). B200 runs FP64 at half the FP32 rate, so 7 against 19 is three
+// quarters of the arithmetic, and the spectra in memory fall from 19 x 8 to 4 x 16
+// bytes per point.
 //
 // Non-negative inputs are centred, a = a' + C u, b = b' + C u (C = 2^B, u the
 // all-ones polynomial):
@@ -41,7 +44,7 @@
 namespace gfb
 {
 
-constexpr int EXACT_MAX_LIMBS = 3;
+constexpr int EXACT_MAX_LIMBS = 4;
 
 struct ExactArgs
 {
@@ -101,10 +104,11 @@ struct ExactErr
         e = max(e, __double2hiint(fabs(d)));
         big = max(big, __double2hiint(fabs(v)));
     }
-    // above 2^50 the distance no longer certifies anything (group_error)
+    // exact_plan keeps in-range rows at or below 2^48; from 2^49 on (coefficients out
+    // of range) the error nears 0.5 and the distance no longer certifies anything
     __device__ __forceinline__ float value() const
     {
-        if (big >= 0x43100000) return 1.0f;
+        if (big >= 0x43000000) return 1.0f;
         return e == 0 ? 0.f : fminf((float)__hiloint2double(e, -1), 0.5f); // rounded up; a distance is at most 0.5
     }
 };

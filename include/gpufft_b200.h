@@ -343,12 +343,18 @@ size_t gpufft_negacyclic_mul_split_workspace_bytes(int n_power, int batch, int n
  *
  * How it is computed. The plan names what the call must hold: FP32 transforms
  * of num_limbs limbs of both operands. On B200 the same integers are cheaper on
- * FP64 transforms with only `a` cut into one to three limbs (5 transforms
- * instead of 19 for 24 bits), so a call whose plan is within the error model
- * runs that way (rings N = 2^5 .. 2^17; from 2^14 on, waves of at least one
- * 2048-point tile per SM; a 16-byte aligned workspace that also holds the
- * FP64 twiddles, 40 N/2 bytes; results apart from the operands), and max_error
- * reports its groups. Other calls run the FP32 limb chain.
+ * FP64 transforms with only `a` cut into one to four limbs (7 transforms
+ * instead of 19 for 24 bits at N = 2^16), so a call whose plan is within the
+ * error model runs that way (rings N = 2^5 .. 2^17; from 2^14 on, waves of at
+ * least one 2048-point tile per SM; a 16-byte aligned workspace that also holds
+ * the FP64 twiddles, 40 N/2 bytes; results apart from the operands), and
+ * max_error reports its groups. Other calls run the FP32 limb chain.
+ *
+ * Rows whose coefficients add up (constant, zero, zero-padded). The FP64 form
+ * takes as many limbs as hold every row of in-range coefficients: N 2^t 2^B (t
+ * bits of `a` in a limb, B bits of `b`, three times that for non-negative inputs)
+ * stays below 2^48. The limb chain's plan is for uniform rows; it may lose such
+ * rows, and then reports 0.5 or 1.0.
  *
  * What max_error certifies. Every result coefficient is exact when the
  * floating-point error of every limb-group value is below 0.5. max_error
@@ -359,16 +365,17 @@ size_t gpufft_negacyclic_mul_split_workspace_bytes(int n_power, int batch, int n
  * above 0.5, so exactness is statistical: the limb plan (gpufft_split_plan)
  * keeps the predicted largest error at or below 0.2, from an error model
  * calibrated on measured limb products (the FP64 form at or below 0.06), and
- * the measured max_error on uniform 24-bit data is about 0.01 at N = 2^16 (0.13
- * in the FP32 chain). Group values above 2^22 (2^50 in the FP64 form) report 1.0
- * (not certified). */
+ * the measured max_error on uniform 24-bit data is below 0.001 at N = 2^16 (0.13
+ * in the FP32 chain). On coherent rows the FP64 form's errors were measured at
+ * most 2^-50 of the bound above, 0.25 (largest seen 0.19). Group values above
+ * 2^22 (2^49 in the FP64 form) report 1.0 (not certified). */
 int gpufft_negacyclic_mul_split_f32(const int32_t* a, const int32_t* b, int64_t* c, int n_power, int batch,
                                     int input_bits, int non_negative, int limb_bits, int num_limbs,
                                     const void* tables, void* workspace, size_t workspace_bytes,
                                     float* max_error, gpufft_stream_t stream);
 /* The FP64 form above (on = 1, the default) or always the chain of limb passes
- * (on = 0); the integers are the same. A negative value only queries. Returns
- * the previous setting. Process-wide. */
+ * (on = 0); the integers are the same wherever the chain reports below 0.5. A
+ * negative value only queries. Returns the previous setting. Process-wide. */
 int gpufft_set_split_tile(int on);
 /* Bounded waits of the exact product that ran out: its kernels have none, so the
  * count is 0. */

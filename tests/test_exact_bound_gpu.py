@@ -1,0 +1,51 @@
+"""GPU tests of what the exact product holds on rows whose coefficients add up
+(constant, half-range, zero and zero-padded operands): the number of limbs has to
+follow the largest magnitude such rows give a limb's product,
+    N 2^top 2^B,  three times that for centred (non-negative) inputs,
+whatever the ring, the width and the sign. Sets whose one-limb or two-limb product
+would pass 2^48, where an FP64 transform's error nears 0.5."""
+import pytest
+import torch
+
+from test_exact_gpu import exact
+
+pytestmark = pytest.mark.gpu
+
+
+def operands(kind, n, batch, bits, nonneg, dev):
+    top = (1 << bits) - 1
+    half = 1 << (bits - 1)
+    a = torch.zeros(batch, n, dtype=torch.int32, device=dev)
+    b = torch.zeros(batch, n, dtype=torch.int32, device=dev)
+    if kind == "max":
+        a.fill_(top)
+        b.fill_(top)
+    elif kind == "halfrange":
+        a.fill_(half)
+        b.fill_(half)
+    elif kind == "padded":
+        a[:, : n // 2] = top
+        b[:, : n // 2] = top
+    elif kind == "padded60":
+        a[:, : n // 2] = int(0.6 * top)
+        b[:, : n // 2] = int(0.6 * top)
+    elif kind == "low":
+        a.fill_(0 if nonneg else -top)
+        b.fill_(top)
+    elif kind == "steps":  # a linear ramp against its reverse
+        r = torch.linspace(0 if nonneg else -top, top, n, device=dev, dtype=torch.float64).round().to(torch.int32)
+        a[:] = r
+        b[:] = r.flip(0)
+    return a, b
+
+
+@pytest.mark.parametrize("n_power,batch,bits,nonneg", [
+    (16, 10, 17, True), (16, 10, 18, False), (14, 38, 19, False), (13, 9, 19, True), (12, 40, 20, True),
+    (10, 64, 20, False), (16, 10, 24, True), (15, 19, 24, True), (17, 5, 24, True), (17, 5, 24, False),
+    (14, 38, 26, True), (13, 40, 27, False), (12, 40, 28, True), (9, 64, 30, True)])
+@pytest.mark.parametrize("kind", ["max", "halfrange", "padded", "padded60", "low", "steps"])
+def test_exact_holds_coherent_rows(gf, dev, n_power, batch, bits, nonneg, kind):
+    a, b = operands(kind, 1 << n_power, batch, bits, nonneg, dev)
+    c, e = gf.negacyclic_mul_split(a, b, input_bits=bits, non_negative=nonneg, return_error=True)
+    assert torch.equal(c, exact(a, b))
+    assert float(e.item()) < 0.5
