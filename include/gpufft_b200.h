@@ -383,8 +383,9 @@ int gpufft_split_wait_timeouts(unsigned* count, int clear);
 /* The same exact product with FP64 transforms, N = 2^2 .. 2^17 (no reference
  * counterpart). Its limb plan uses the FP64 error model, so it needs far fewer
  * limbs (two 12-bit limbs for 24-bit coefficients at N = 2^16). `tables` is the
- * f64 native twiddle block (gpufft_ffnt_make_tables_f64). Runs in the form
- * described above where it applies (one operand whole). */
+ * f64 native twiddle block (gpufft_ffnt_make_tables_f64). Plans of one limb run
+ * in the form described above where it applies; plans of more limbs cut both
+ * operands, as given, and leave an error of about 3e-6 (24 bits, N = 2^16). */
 int gpufft_split_plan_f64(int n_power, int input_bits, int non_negative, int* limb_bits, int* num_limbs);
 size_t gpufft_negacyclic_mul_split_f64_workspace_bytes(int n_power, int batch, int num_limbs);
 int gpufft_negacyclic_mul_split_f64(const int32_t* a, const int32_t* b, int64_t* c, int n_power, int batch,

@@ -3,11 +3,12 @@
 follow the largest magnitude such rows give a limb's product,
     N 2^top 2^B,  three times that for centred (non-negative) inputs,
 whatever the ring, the width and the sign. Sets whose one-limb or two-limb product
-would pass 2^48, where an FP64 transform's error nears 0.5."""
+would pass 2^48, where an FP64 transform's error nears 0.5. And what calls with FP64
+tables report."""
 import pytest
 import torch
 
-from test_exact_gpu import exact
+from test_exact_gpu import exact, rows
 
 pytestmark = pytest.mark.gpu
 
@@ -49,3 +50,23 @@ def test_exact_holds_coherent_rows(gf, dev, n_power, batch, bits, nonneg, kind):
     c, e = gf.negacyclic_mul_split(a, b, input_bits=bits, non_negative=nonneg, return_error=True)
     assert torch.equal(c, exact(a, b))
     assert float(e.item()) < 0.5
+
+
+@pytest.mark.parametrize("n_power,batch,bits,nonneg", [
+    (16, 10, 24, True), (14, 38, 22, True), (13, 40, 24, False), (10, 64, 24, True),  # two limbs
+    (16, 10, 16, False), (13, 40, 16, False), (11, 64, 18, True)])                    # one limb
+def test_f64_plan_keeps_its_error(gf, dev, n_power, batch, bits, nonneg):
+    # calls with FP64 tables report what their own limb plan leaves: the plan's passes
+    # and the form with b whole differ at most by the order of roundings (a maximum
+    # over batch N values moves by less than a factor of two)
+    a, b = rows(gf, dev, 1 << n_power, batch, bits, nonneg, n_power + bits)
+    kw = dict(input_bits=bits, non_negative=nonneg, precision="f64", return_error=True)
+    prev = gf.set_split_tile(0)
+    try:
+        c0, e0 = gf.negacyclic_mul_split(a, b, **kw)
+        gf.set_split_tile(1)
+        c1, e1 = gf.negacyclic_mul_split(a, b, **kw)
+    finally:
+        gf.set_split_tile(prev)
+    assert torch.equal(c0, c1) and torch.equal(c1, exact(a, b))
+    assert float(e1.item()) <= 2 * float(e0.item())
