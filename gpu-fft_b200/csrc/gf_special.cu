@@ -88,23 +88,30 @@ __device__ __forceinline__ void special_network(cx<T> (&x)[1 << L], const cx<T> 
 }
 
 // A pass of spans 2^p0 .. 2^(p0+L-1) (p0 > 0), one column per thread, in the vectors
-// blockIdx.y, blockIdx.y + gridDim.y, ...: a column's twiddles are its own (as many
-// bytes as its points) but the same in every vector.
-template <typename T, int L, bool FWD>
+// v, v + stride, ...: a column's twiddles are its own (as many bytes as its points)
+// but the same in every vector. The lanes of a CTA are 128 columns of one vector, or
+// (SHARED) all the columns of several neighbouring vectors that have fewer (2^10
+// points and below). One such vector to a CTA leaves 112 of 128 lanes idle at 2^6 ..
+// 2^8 points: 20000 vectors of 2^8, FP64, this pass 39 us against 25.
+template <typename T, int L, bool FWD, bool SHARED>
 __global__ void __launch_bounds__(SPECIAL_THREADS) special_col_kernel(const SpecialArgs<T> a)
 {
     pdl_begin(); // before any global-memory access (programmatic launch)
     constexpr int R = 1 << L;
-    const long long idx = (long long)blockIdx.x * SPECIAL_THREADS + threadIdx.x;
     const int m = a.m, p0 = a.p0;
+    const int lc = m - L; // log2 of a vector's columns
+    const long long idx =
+        SHARED ? threadIdx.x & ((1 << lc) - 1) : (long long)blockIdx.x * SPECIAL_THREADS + threadIdx.x;
     const long long lo = idx & ((1LL << p0) - 1);
     const long long hi = idx >> p0;
-    if (hi >= (1LL << (m - p0 - L))) return;
+    if (!SHARED && hi >= (1LL << (m - p0 - L))) return;
+    const long long first = SHARED ? (long long)blockIdx.y * (SPECIAL_THREADS >> lc) + (threadIdx.x >> lc) : blockIdx.y;
+    const long long stride = SHARED ? (long long)gridDim.y * (SPECIAL_THREADS >> lc) : gridDim.y;
     cx<T>* p = a.data + (hi << (p0 + L)) + lo;
     cx<T> w[R - 1];
     special_twiddles<T, L>(w, a, lo);
 #pragma unroll 1
-    for (long long b = blockIdx.y; b < a.batch; b += gridDim.y)
+    for (long long b = first; b < a.batch; b += stride)
     {
         cx<T>* q = p + (b << m);
         cx<T> x[R];
@@ -386,12 +393,21 @@ template <typename T, bool FWD> static int launch_special_pass(const SpecialArgs
                             dim3(SPECIAL_THREADS), 0, s, a);
         }
         // vectors per thread: as many as leave two CTAs' worth of columns per slot
-        // (three CTAs per SM in FP64, five in FP32)
-        const long long bx = ((1LL << (a.m - LL)) + SPECIAL_THREADS - 1) / SPECIAL_THREADS;
-        const long long want = (long long)sm_count() * (sizeof(T) == 8 ? 6 : 10);
-        const long long per = std::min<long long>(8, std::max<long long>(1, bx * a.batch / want));
-        const long long by = std::min<long long>(65535, (a.batch + per - 1) / per);
-        return launch_k(special_col_kernel<T, LL, FWD>, dim3((unsigned)bx, (unsigned)by), dim3(SPECIAL_THREADS), 0, s, a);
+        // (three CTAs per SM in FP64, five in FP32). Two and three FP64 spans of short
+        // vectors want four and two times as many (50000 vectors of 2^6: 28.6 us with
+        // 888 CTAs, 25.1 with 3552); FP32 and single spans lose by that, bound by the
+        // launch of their CTAs (10000 vectors of 2^9, FP32: 28.5 against 40.9).
+        const bool shared = a.m - LL < 7;
+        const long long bx = shared ? 1 : 1LL << (a.m - LL - 7);
+        const int vectors = shared ? SPECIAL_THREADS >> (a.m - LL) : 1; // of a CTA at a time
+        const long long rows = (a.batch + vectors - 1) / vectors;
+        const long long want = ((long long)sm_count() * (sizeof(T) == 8 ? 6 : 10))
+                               << (shared && sizeof(T) == 8 && LL > 1 ? 4 - LL : 0);
+        const long long per = std::min<long long>(8, std::max<long long>(1, bx * rows / want));
+        const long long by = std::min<long long>(65535, (rows + per - 1) / per);
+        const dim3 grid((unsigned)bx, (unsigned)by);
+        return shared ? launch_k(special_col_kernel<T, LL, FWD, true>, grid, dim3(SPECIAL_THREADS), 0, s, a)
+                      : launch_k(special_col_kernel<T, LL, FWD, false>, grid, dim3(SPECIAL_THREADS), 0, s, a);
     });
 }
 
