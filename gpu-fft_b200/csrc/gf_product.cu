@@ -231,12 +231,12 @@ constexpr int NATIVE_MAX_NPOWER = 22; // two-pass plans: M = N/2 <= 2^21
 constexpr size_t WAVE_TARGET_BYTES = 80ull << 20;
 constexpr size_t WAVE_TILE_BYTES = 320ull << 20;
 
-static long long wave_products(int n_power, long long batch, size_t cx_bytes)
+static long long wave_products(int n_power, long long batch, size_t cx_bytes, size_t tile_bytes = WAVE_TILE_BYTES)
 {
     const int m = n_power - 1;
     if (m <= EBITS) return batch;
     const size_t per = 2 * ((size_t)1 << m) * cx_bytes;
-    long long w = (long long)((m - TILE_LT <= TILE_MAX_L ? WAVE_TILE_BYTES : WAVE_TARGET_BYTES) / per);
+    long long w = (long long)((m - TILE_LT <= TILE_MAX_L ? tile_bytes : WAVE_TARGET_BYTES) / per);
     if (w < 1) w = 1;
     w = round_wave(w, ((long long)1 << m) / ECTA);
     return w < batch ? w : batch;
@@ -526,7 +526,11 @@ namespace gfb
 static long long host_chunk(int n_power, long long batch, long long chunk, size_t cxb)
 {
     if (chunk > 0) return chunk < batch ? chunk : batch;
-    return pipe_chunk(wave_products(n_power, batch, cxb), batch);
+    // three slots of a, b and c come with every chunk, and the transfers bound the
+    // call (N = 2^16, FP64, 1184 products: chunks of 37 / 74 / 111 / 148 products take
+    // 25.6 / 25.3 / 25.1 / 25.6 ms and 203 / 407 / 610 / 814 MiB): chunks stay at 80 MiB
+    // of spectra, where the device product's waves do not
+    return pipe_chunk(wave_products(n_power, batch, cxb, WAVE_TARGET_BYTES), batch);
 }
 
 template <typename T>
