@@ -116,16 +116,24 @@ template <int K> static int launch_exact_tile(const ExactArgs& a, int m, cudaStr
     return launch_k(exact_tile<K>, dim3((unsigned)tiles), dim3(tile::HT), EXACT_SMEM, s, a, m);
 }
 
-template <int m, int K> static int launch_exact_single(const ExactArgs& a, cudaStream_t s)
+template <int m, int K, int BLOCKS> static int launch_exact_single_b(const ExactArgs& a, long long ctas, cudaStream_t s)
 {
     using tl = TileOf<m == 12 ? 12 : 11>;
     static int done[64] = {0};
     const size_t smem = (size_t)(tl::SLOT + tl::TWN) * sizeof(cx<double>);
-    const int st = ensure_smem(exact_single<m, K>, smem, done);
+    const int st = ensure_smem(exact_single<m, K, BLOCKS>, smem, done);
     if (st) return st;
-    const long long ctas = ((a.W << m) + tl::P - 1) / tl::P;
     GF_TRACE(tr, (double)(a.W << m) * (2 * 2 * 4 + 2 * 8), s, "exact_single<L%d,k%d>", m, K);
-    return launch_k(exact_single<m, K>, dim3((unsigned)ctas), dim3(tl::HT), smem, s, a);
+    return launch_k(exact_single<m, K, BLOCKS>, dim3((unsigned)ctas), dim3(tl::HT), smem, s, a);
+}
+
+template <int m, int K> static int launch_exact_single(const ExactArgs& a, cudaStream_t s)
+{
+    using tl = TileOf<m == 12 ? 12 : 11>;
+    const long long ctas = ((a.W << m) + tl::P - 1) / tl::P;
+    const bool two = K > 1 && (ctas <= 2LL * sm_count() || (K > 2 && ctas > 3LL * sm_count()));
+    return two ? launch_exact_single_b<m, K, exact_single_blocks<m>(true)>(a, ctas, s)
+               : launch_exact_single_b<m, K, exact_single_blocks<m>(false)>(a, ctas, s);
 }
 
 int split_exact(const int32_t* a, const int32_t* b, int64_t* c, int m, int batch, int input_bits, bool non_negative,

@@ -364,9 +364,9 @@ template <int K> __global__ void __launch_bounds__(tile::HT, tile_min_blocks<dou
 // threads, one of 4096 points to a CTA of 256
 // ---------------------------------------------------------------------------
 // Two CTAs per SM (one at 4096 points) where a thread holds 16 twist factors of its
-// own; three below, where they repeat.
-template <int m, int K>
-__global__ void __launch_bounds__(m == 12 ? 256 : 128, m == 12 ? 1 : m == 11 ? 2 : 3) exact_single(const ExactArgs a)
+// own; three below, where they repeat (BLOCKS, exact_single_blocks).
+template <int m, int K, int BLOCKS>
+__global__ void __launch_bounds__(m == 12 ? 256 : 128, BLOCKS) exact_single(const ExactArgs a)
 {
     pdl_begin(); // before any global-memory access (programmatic launch)
     using tl = TileOf<m == 12 ? 12 : 11>;
@@ -460,6 +460,17 @@ __global__ void __launch_bounds__(m == 12 ? 256 : 128, m == 12 ? 1 : m == 11 ? 2
         }
     }
     report_err(a.max_err, err.value());
+}
+
+// CTAs per SM that exact_single is compiled for. 1024 points: at three, several limbs
+// spill (two limbs 290 bytes a thread, three 520), so a launch that two per SM hold
+// takes two (N = 2^11, 24 bits, 2 / 40 / 400 products: 19 / 19 / 31 us against 27 / 28 /
+// 34), and one that three hold takes three (800: 41 against 51). Beyond, two limbs
+// take three (4000: 160 against 173) and more limbs two (28 bits, 1200 / 4000: 103 / 261
+// against 108 / 281).
+template <int m> constexpr int exact_single_blocks(bool two)
+{
+    return m == 12 ? 1 : m == 11 || (m == 10 && two) ? 2 : 3;
 }
 
 } // namespace gfb

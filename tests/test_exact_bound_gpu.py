@@ -70,3 +70,38 @@ def test_f64_plan_keeps_its_error(gf, dev, n_power, batch, bits, nonneg):
         gf.set_split_tile(prev)
     assert torch.equal(c0, c1) and torch.equal(c1, exact(a, b))
     assert float(e1.item()) <= 2 * float(e0.item())
+
+
+@pytest.mark.parametrize("batch,bits", [(1, 24), (296, 24), (592, 24), (593, 24), (1201, 24), (2, 26), (701, 26), (889, 26), (3, 28)])
+def test_exact_2e11_ctas_per_sm(gf, dev, batch, bits):
+    # two or three CTAs per SM by the number of limbs and CTAs (two products each)
+    a, b = rows(gf, dev, 1 << 11, batch, bits, True, batch + bits)
+    a[0, 1024:] = 0
+    c, e = gf.negacyclic_mul_split(a, b, input_bits=bits, non_negative=True, return_error=True)
+    assert float(e.item()) < 0.5 and torch.equal(c, exact(a, b))
+
+
+def test_exact_2e11_few_products_not_slower_than_the_chain(gf, dev):
+    # two products of N = 2^11, 24 bits: 19 us against the limb chain's 21.6 (27 where
+    # the one-kernel form spills for a third CTA per SM); sides in turn, best of many
+    a, b = rows(gf, dev, 1 << 11, 2, 24, True, 5)
+    tables = gf.ffnt_tables(11, "f32")
+    out = torch.empty(a.shape, dtype=torch.int64, device=dev)
+    ws = torch.empty(1 << 22, dtype=torch.uint8, device=dev)
+    best = {}
+    try:
+        for _ in range(15):
+            for on in (1, 0):
+                gf.set_split_tile(on)
+                t0, t1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+                for k in range(40):
+                    if k == 10:
+                        t0.record()
+                    gf.negacyclic_mul_split(a, b, out=out, input_bits=24, non_negative=True, tables=tables, workspace=ws)
+                t1.record()
+                torch.cuda.synchronize()
+                t = t0.elapsed_time(t1)
+                best[on] = min(t, best.get(on, t))
+    finally:
+        gf.set_split_tile(1)
+    assert best[1] <= 1.05 * best[0]
