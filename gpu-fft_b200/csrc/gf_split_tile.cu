@@ -145,8 +145,11 @@ int split_exact(const int32_t* a, const int32_t* b, int64_t* c, int m, int batch
     int w = 0, K = 0;
     if (!exact_plan(m + 1, B, non_negative, &w, &K)) return -1;
     const bool single = m <= 12;
-    // one CTA runs its product's transforms in turn: few 4096-point ones take the
-    // chain, which spreads them (one product of 24 bits: 24.6 against 31.2 us)
+    // one CTA runs its product's transforms in turn: up to 16 products of 4096-point
+    // ones take the chain, which spreads them (16 products, two limbs 28.1 us against
+    // 33.3, three 28.0 against 54). The chain stays ahead up to 30 products with two
+    // limbs and 72 with three, but it does not hold every row (exact_plan): from 17 on
+    // calls keep the form that does.
     if (m == 12 && K > 1 && batch <= 16) return -1;
     // the result is written while operands are still read
     const size_t in = (size_t)batch * 2 * M * sizeof(int32_t);
@@ -161,7 +164,10 @@ int split_exact(const int32_t* a, const int32_t* b, int64_t* c, int m, int batch
     if (ws_bytes < tab + per) return -1;
     long long W = single ? batch : (long long)((ws_bytes - tab) / per);
     if (W > batch) W = batch;
-    // a wave with fewer tiles than SMs takes the chain of FP32 passes
+    // a wave with fewer tiles than SMs takes the limb chain (N = 2^16; at the line, ten
+    // products, the two forms: one limb 26.5 against 46.5 us, two 42.0 / 46.5, three
+    // 53.3 / 54.8; below it, four products: 21.7 / 33.6, 37.5 / 33.9, 48.0 / 37.5). One
+    // limb would win there too; four lose up to six products of N = 2^17 (73 / 69 us).
     if (!single && (W << (m - 11)) < (long long)sm_count()) return -1;
     if (tables)
     {

@@ -32,10 +32,10 @@
 // Rings N = 2^5 .. 2^13 run in one kernel, exact_single, a CTA holding whole
 // products.
 //
-// Measured (B200): N = 2^16, batch 256, 24 bits: 413 us (columns 109 + 85, tiles
-// 222, tables 3) where five FP32 limbs of both operands on shared-memory tiles took
-// 824; N = 2^13, batch 333, 16 bits: 40 us against 360; N = 2^12, batch 2000, 16
-// bits: 87 against 809; one product of N = 2^12: 19 against 24.
+// Measured (B200) against the limb chain: N = 2^16, batch 256, 24 bits, three limbs:
+// 516 us (columns 126 + 110, tiles 296, tables 7) against 1076; 16 bits, one limb: 230
+// against 867; N = 2^13, batch 333, 16 bits: 39 against 378; N = 2^12, batch 2000, 16
+// bits: 77 against 809; one product of N = 2^12, 24 bits: 19 against 21.5.
 #pragma once
 
 #include "gf_split.cuh"
@@ -317,7 +317,7 @@ template <int K> __global__ void __launch_bounds__(tile::HT, tile_min_blocks<dou
     const long long base = ((long long)blockIdx.x << 11) + t; // flat over the products
     const long long g = (long long)blockIdx.x & ((1LL << (m - 11)) - 1);
     const long long WM = a.W * M;
-    if (t == 0) // the other limbs wait in L2 (N = 2^16, batch 256, 24 bits: 437 -> 431 us)
+    if (t == 0) // the other limbs wait in L2 (N = 2^16, batch 256, two limbs: 437 -> 431 us)
     {
 #pragma unroll
         for (int l = 1; l < K; l++) prefetch_l2(a.spec + l * WM + base, tile::P * sizeof(cx<double>));
@@ -332,9 +332,11 @@ template <int K> __global__ void __launch_bounds__(tile::HT, tile_min_blocks<dou
     tile::forward<double>(pk, sm, tw, t);
     __syncthreads(); // the parked operand's last transpose is read
     // U of the thread's points j = 2048 g + 16 t + r: coalesced in the permuted order
-    const cx<double>* up = a.uspec + (m > EBITS ? ((g >> 1) << EBITS) + ((g & 1) << 7) + t : (g << 11) + 16 * t);
-    const int us = m > EBITS ? 256 : 1;
-#pragma unroll
+    // (m > 12 here)
+    const cx<double>* up = a.uspec + ((g >> 1) << EBITS) + ((g & 1) << 7) + t;
+    // a loop: unrolled, three limbs spilled and waited for instructions (0.74 of the
+    // stalls per issue; N = 2^16, 24 bits, batch 256: 324 -> 296 us, two limbs 212 -> 199)
+#pragma unroll 1
     for (int l = 0; l < K; l++)
     {
         if (l > 0)
@@ -351,7 +353,7 @@ template <int K> __global__ void __launch_bounds__(tile::HT, tile_min_blocks<dou
         else
         {
 #pragma unroll
-            for (int r = 0; r < R; r++) x[r] = exact_product(x[r], pk[r], a, __ldg(&up[r * us].y), l == K - 1);
+            for (int r = 0; r < R; r++) x[r] = exact_product(x[r], pk[r], a, __ldg(&up[r * 256].y), l == K - 1);
         }
         tile::inverse<double>(x, sm, tw, t);
 #pragma unroll
