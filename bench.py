@@ -601,8 +601,8 @@ def time_path(step, host_step, a, b, c, hosts, args, stream, torch, barrier, max
 # launch, so traffic per launch = ratio x the kernel's tagged bytes per launch.
 NCU_TRAFFIC = {
     # 128 products (2048 tiles of 2048 points), DRAM rate x duration of the capture:
-    # 281.6 MB of 335.5 MB tagged
-    "split_tile<f64,k2>": (281.6 / 335.5, "ncu capture of a 128-product launch"),
+    # 430.3 MB of 469.8 MB tagged
+    "split_tile<f64,k3>": (430.3 / 469.8, "ncu capture of a 128-product launch"),
     # 157.3 MB of 201.3 MB tagged
     "tile_product<f64,mul>": (157.3 / 201.3, "ncu capture of a 128-product launch"),
     # 211.5 MB of 268.4 MB tagged
@@ -1089,7 +1089,8 @@ def main():
                                  traced_launches=sum(r["launches"] for r in rows),
                                  value=world * batch / (ms * 1e-3), achieved=achieved,
                                  h2d=2 * batch * n * a_host.element_size(), d2h=batch * n * c_host.element_size(),
-                                 dtype="f64" if name in ("f64", "dropin_f64", "split64") else "f32",
+                                 # the exact product's transforms are FP64 whichever tables it is given
+                                 dtype="f32" if name == "f32" else "f64",
                                  c=c[:2].cpu() if rank == 0 else None)
             del a, b, c, a_host, b_host, c_host
         time.sleep(0.3)

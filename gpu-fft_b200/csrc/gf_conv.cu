@@ -13,7 +13,8 @@
 // products G conj(B) and G conj(A), two inverse transforms, and only the real
 // parts (the coefficients below N) are written.
 //
-//   2N <= 8192:  one kernel per product group (vjp_kernel<L, true>);
+//   2N <= 8192:  one kernel (single_kernel, SINGLE_VJP, from 2N = 32 on; results
+//                over operands and 2N < 32: vjp_kernel<L, true>);
 //   otherwise:   strided first forward pass of g, a, b (pass_kernel, IN_VJP3),
 //                contiguous middle pass (tile_product_kernel, TILE_VJP, from two
 //                2048-point tiles per SM on; vjp_kernel<12, false> below that),
@@ -131,8 +132,8 @@ static long long vjp_wave(int m, long long batch)
 {
     if (m <= EBITS) return batch;
     // one launch per phase over as many rows as fit 320 MiB of spectra for the
-    // tile kernel's rings (512 rows of N = 2^14, all kernels of the call: four
-    // waves of 128 with the 4096-point middle pass 368 us, one with the tile kernel 187 us)
+    // tile kernel's rings (512 rows of N = 2^14, 192 MiB: workspaces of 24 / 48 / 96 /
+    // 192 MiB 233 / 180 / 183 / 177 us; with the 4096-point middle pass 335, and 311 from 48 MiB on)
     const size_t per = 3 * ((size_t)1 << m) * sizeof(cx<float>);
     long long w = (long long)((m - TILE_LT <= TILE_MAX_L ? 320ull << 20 : 48ull << 20) / per);
     if (w < 1) w = 1;

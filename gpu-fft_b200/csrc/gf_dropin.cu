@@ -18,11 +18,11 @@ namespace gfb
 
 // Passes of (m - 11, 11) stages, the second on 2048-point tiles, where a column pass
 // (FP64, up to 2^16 points) or any first pass (FP32, up to 2^20: C_C N = 2^20, batch
-// 11, 319 us against 353; FP64 328 against 306 at batch 5) has a kernel for the rest
-// and two tiles per SM keep the tile pass's CTAs overlapping; the plan above
-// otherwise. FP64 FFNT calls (fold) keep 4096-point
-// tiles from three per two SMs on: one column stage fewer next to the fold, longer
-// runs under one staging of the twiddles (product, N = 2^16: batch 256 351 against
+// 11, both plans on one GPU: 319 us against 353; FP64 328 against 306 at batch 5) has a
+// kernel for the rest and two tiles per SM keep the tile pass's CTAs overlapping; the
+// plan above otherwise. FP64 FFNT calls (fold) keep 4096-point tiles from three per two
+// SMs on: one column stage fewer next to the fold, longer runs under one staging of the
+// twiddles (product, N = 2^16: batch 256 351 against
 // 413 us, batch 30 52 against 59; N = 2^15, batch 20, below the line: 36 against 34;
 // C_C N = 2^14, batch 100: 83 against 80, R_R, batch 75: 56 against 51).
 template <typename T> static Plan transform_plan(int m, long long batch, bool fold)

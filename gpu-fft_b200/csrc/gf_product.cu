@@ -5,16 +5,17 @@
 // unfold: reference fft.cu:1013-1384, fft_cpu.cu:301-432) fused so that the
 // two spectra are never written out as a caller-visible intermediate:
 //
-//   N <= 8192:  one kernel. A CTA loads both operands of 4096/(N/2) products,
-//               runs every forward stage on both in registers (shared twiddles
-//               and index arithmetic), multiplies, runs every inverse stage,
-//               untwists and writes the real product: one HBM read of a and b
-//               and one HBM write of c.
+//   N <= 8192:  one kernel (single_kernel from N = 32 on, fused_kernel below; few
+//               products of N >= 2048 on thread-block clusters). A CTA transforms
+//               one operand and parks it in registers, then transforms the other,
+//               multiplies, runs every inverse stage, untwists and writes the real
+//               product: one HBM read of a and b and one HBM write of c.
 //   N > 8192:   three kernels per wave of products -- the first forward pass
-//               (strided, fold+twist fused into the load), the fused last pass
-//               (forward both, multiply, inverse, in registers) and the last
-//               inverse pass (strided, scale+untwist+unfold fused into the
-//               store). The two spectra of a wave live in a caller-provided
+//               (strided, fold+twist fused into the load), the middle
+//               (tile_product_kernel on 2048-point tiles, or the fused 4096-point
+//               pass where a wave has few tiles: forward both, multiply, inverse)
+//               and the last inverse pass (strided, scale+untwist+unfold fused into
+//               the store). The two spectra of a wave live in a caller-provided
 //               workspace; its size sets the wave (products per launch).
 //
 // Twiddles come from gpufft_ffnt_make_tables_*, generated on the device with
@@ -186,9 +187,10 @@ template <typename T, bool SINGLE> static int launch_fused(const FusedArgs<T>& a
 // kernel's CTAs too few to overlap: they take the middle pass (FP64, N = 2^16, at the
 // line, 20 products: 26.7 us on tiles, 34.2 with the middle pass).
 // FP64 negacyclic waves of four to five tiles per SM also take the middle pass, though
-// the tiles are faster there (N = 2^16, 40 products: 44 against 53 us): programs that
-// read the trace rely on its rows for such a wave (three column stages, one
-// fused_r8_kernel launch, their bytes).
+// the tiles are faster there (N = 2^16, 40 products: 44 against 53 us), as they did
+// before there were tiles: the trace's test reads that pass's rows (three column
+// stages, one fused_r8_kernel launch) from 40 products of N = 2^16. Nothing else needs
+// the line.
 template <typename T> static Plan product_plan(int m, long long w, bool negacyclic)
 {
     Plan p = make_plan(m);
@@ -225,9 +227,13 @@ constexpr int NATIVE_MIN_NPOWER = 2;
 constexpr int NATIVE_MAX_NPOWER = 22; // two-pass plans: M = N/2 <= 2^21
 // Recommended wave, then rounded to whole waves of the SMs. Rings of the tile
 // kernel: up to 320 MiB of spectra, as every launch ends in a partial wave of CTAs
-// (N = 2^16, 1 MiB per product, batch 256, FP64: 74 / 111 / 256 products per wave
-// run 252 / 252 / 241 us). Larger rings keep 80 MiB (the 4096-point middle pass at
-// N = 2^16: 37 / 74 / 256 products ran 290 / 286 / 302 us).
+// (FP64, 2^24 coefficients per operand, workspaces of 80 / 160 / 320 MiB in turn on one
+// GPU, three repeats within 1 %: N = 2^14 230 / 231 / 229 us, 2^15 242 / 239 / 236, 2^16
+// 260 / 255 / 247, 2^17 272 / 265 / 258, 2^18 313 / 291 / 275; on another 2^16 took 267 /
+// 256 / 254. FP32, 2^14 .. 2^18: 115 / 116 / 117 / 135 / 143 at 80 MiB, 112 / 115 / 120 /
+// 136 / 143 at 320). A smaller workspace costs no more than that. Larger rings keep
+// 80 MiB (the 4096-point middle pass at N = 2^16: 37 / 74 / 256 products ran 289 / 287 /
+// 302 us).
 constexpr size_t WAVE_TARGET_BYTES = 80ull << 20;
 constexpr size_t WAVE_TILE_BYTES = 320ull << 20;
 

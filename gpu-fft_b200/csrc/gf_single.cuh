@@ -11,10 +11,10 @@
 // transform and store phases did not overlap, and read the innermost twiddles from
 // the table at a stride of 128 bytes. Values have its bits.
 //
-// Measured (B200, start -> here): negacyclic N = 2^11, batch 4000: FP64 156 -> 64 us
-// (47 % of the HBM rate on operands and result), FP32 78 -> 37; N = 2^13, batch 500
-// FP64 94 -> 49; cyclic 2^10, batch 4000 FP64 99 -> 57; adjoint N = 2^12, batch
-// 1000: 231 -> 109 with the forward product.
+// Measured (B200, the engine's form -> this one): negacyclic N = 2^11, batch 4000:
+// FP64 156 -> 64 us (47 % of the HBM rate on operands and result), FP32 78 -> 37;
+// N = 2^13, batch 500, FP64 94 -> 49; cyclic 2^10, batch 4000, FP64 99 -> 57; adjoint
+// N = 2^12, batch 1000: 231 -> 109 with the forward product.
 #pragma once
 
 #include "gf_tile.cuh"

@@ -28,7 +28,12 @@
 //   split_inv0_col / split_inv0   last inverse pass (strided) of every group
 //                with scale, untwist, unfold, rounding and the int64
 //                recombination in registers.
-// N <= 8192 runs all of it in one kernel (split_mid<true>).
+// N <= 8192 runs all of it in one kernel (split_mid<true>) where the batch fills the
+// SMs, or N <= 512.
+//
+// This limb chain is what calls run that the FP64 form with one operand whole
+// (gf_split_tile.cuh) does not take: few products, rings above 2^17, FP64 plans of
+// several limbs, plans outside the error model, results over operands.
 #pragma once
 
 #include <type_traits>
