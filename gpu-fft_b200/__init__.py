@@ -377,8 +377,9 @@ def negacyclic_mul_split(a, b, out=None, input_bits=None, non_negative=None, lim
     """Exact c = a * b mod (X^N + 1) for (batch, N) int32 tensors from a limb plan for
     FP32 (precision="f32", N <= 2^22, float tables) or FP64 (precision="f64", N <= 2^17,
     double tables) transforms; returns an int64 tensor (and the max pre-rounding error).
-    Plans within the error model run on FP64 transforms with b whole where that is
-    faster (include/gpufft_b200.h), which also holds rows whose coefficients add up."""
+    Plans within the error model (double tables: of one limb) run on FP64 transforms
+    with b whole where that applies (include/gpufft_b200.h), which also holds rows whose
+    coefficients add up."""
     import torch
     batch, n = a.shape
     n_power = n.bit_length() - 1
